@@ -210,17 +210,19 @@ def transform_flops_per_launch(N):
 
 
 def fft_bytes_per_launch(N, fp32=False):
-    """Algorithmic bytes of one FFT row pass over the 6 fields of a solve,
-    averaged over the 4 passes: every field's r x c array is read once and
-    written once per pass, and one pass also reads the eigenvalue matrix.
-    float64: 8 bytes per element everywhere (8 + 8, plus 8 / 4 for the
-    eigenvalues). float32 transforms: the first pass reads float64 and
-    writes float32, the last reads float32 and writes float64, the
-    intermediates and eigenvalues are float32 (44 bytes per element over
-    the 4 passes)."""
+    """Algorithmic bytes of one FFT launch over the 6 fields of a solve,
+    averaged over the solve's launches, every field's r x c array read once
+    and written once per launch. float64 (fft64_a/b/d_kernel, 3 launches):
+    8 + 8 bytes an element, 8 more for the eigenvalues in the second, and in
+    the third, which also finalises the step, the previous field read and
+    the average written (the field itself in one solve of two).
+    float32 transforms (fft_rows_kernel, 4 launches): the first reads
+    float64 and writes float32, the last reads float32 and writes float64,
+    the intermediates and eigenvalues are float32 (44 bytes an element over
+    the 4)."""
     M = N - 2
     dims = [(N, M), (M, N), (M, M), (M, N), (N, M), (N, N)]
-    per = 44 / 4 if fp32 else 8 * (2 + 0.25)
+    per = 44 / 4 if fp32 else 8 * (2 + 3 + 3.5) / 3
     return sum(per * r * c for r, c in dims)
 
 
@@ -393,14 +395,17 @@ def run_ours(args, rank, world, dist):
         f32 = args.precision == 'fft32'
         by = fft_bytes_per_launch(N, f32)
         ach = by / (avg_ms * 1e-3) / 1e9
-        roof = {'kernel': f'fft_rows_kernel ({"FP32" if f32 else "FP64"} DST/DCT row-FFT pass, 6 fields)',
+        roof = {'kernel': 'fft_rows_kernel (FP32 DST/DCT row-FFT pass, 6 fields)' if f32
+                else 'fft64_a/b/d_kernel (FP64 DST/DCT, 6 fields, average of the three launches)',
                 'bound': 'hbm',
                 'achieved': ach, 'peak': hbm, 'unit': 'GB/s', 'frac': ach / hbm,
                 'peak_source': hbm_src, 'algorithmic_per_launch': by, 'avg_launch_ms': avg_ms,
                 'traffic': None,
                 'note': ('the rows stay in L2 (ncu: L2 throughput ~0.14 of peak); while active the pass is '
                          'bound by the L1/shared-memory pipe (~0.72 of peak) and by its barrier-separated radix '
-                         'passes: profiles/fft_rows_kernel_641.md')}
+                         'passes: profiles/fft_rows_kernel_641.md') if f32 else
+                        ('the rows stay in L2 (ncu: L2 throughput ~0.11 of peak); bound by latency: FP64 pipe '
+                         '~0.22, issue ~0.27 of peak at 16 warps per SM: profiles/fft64_kernels_641.md')}
     elif dom == 'transform' and stage[dom]['timed']:
         avg_ms = stage[dom]['ms'] / stage[dom]['timed']
         fl = transform_flops_per_launch(N)

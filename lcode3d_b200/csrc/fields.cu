@@ -25,11 +25,8 @@
 
 #include "lc3d_internal.cuh"
 
-#ifndef LC3D_FFT_STREAMS
-#define LC3D_FFT_STREAMS 2   // float64 FFT passes of a solve on 1, 2 or 3 streams
-#endif
 #ifndef LC3D_FFT32_STREAMS
-#define LC3D_FFT32_STREAMS 3   // ... float32 FFT passes
+#define LC3D_FFT32_STREAMS 3   // float32 FFT passes of a solve on 1, 2 or 3 streams
 #endif
 #ifndef LC3D_FIN_PER_GROUP
 #define LC3D_FIN_PER_GROUP 1
@@ -456,12 +453,14 @@ int fields_init(lc3d_ctx* c) {
         LC3D_TRY(upload32(&c->lam32_neu, ln));
     }
     const size_t plane = (size_t)N * N * sizeof(double);
-    const size_t tplane = (size_t)N * fft_pitch(N) * sizeof(double);   // the transform intermediates
+    const size_t tplane = (size_t)N * fft64_pitch(N) * sizeof(double);   // the transform intermediates
     for (int f = 0; f < 6; ++f) {
         LC3D_CUDA_TRY(cudaMalloc(&c->rhs[f], plane));
         LC3D_CUDA_TRY(cudaMalloc(&c->t1[f], tplane));
         LC3D_CUDA_TRY(cudaMalloc(&c->t2[f], tplane));
         LC3D_CUDA_TRY(cudaMalloc(&c->raw[f], plane));
+        LC3D_CUDA_TRY(cudaMemset(c->t1[f], 0, tplane));
+        LC3D_CUDA_TRY(cudaMemset(c->t2[f], 0, tplane));
         LC3D_CUDA_TRY(cudaMemset(c->rhs[f], 0, plane));
         LC3D_CUDA_TRY(cudaMemset(c->raw[f], 0, plane));
     }
@@ -558,6 +557,29 @@ int solve_fields(lc3d_ctx* c, int which, const SolveInputs& in, const SolveOutpu
         LC3D_CUDA_TRY(cudaGetLastError());
     }
 
+    if (c->use_fft && c->p.precision == LC3D_PREC_FP64) {
+        Fft64Desc d[6]{};
+        int cnt = 0;
+        for (int f = 0; f < 6; ++f) {
+            if (!on[f]) continue;
+            const FieldGeom g = geom(c, f);
+            Fft64Desc& e = d[cnt++];
+            e.rhs = c->rhs[f];
+            e.type0 = g.type0;
+            e.type1 = g.type1;
+            e.t1 = c->t1[f];
+            e.t2 = c->t2[f];
+            e.out = o.out[f];
+            if (o.mode == 1) {
+                e.prev = o.prev[f];
+                e.avg = o.avg[f];
+                e.variant_a = c->p.field_solver_variant_A && f != 2 && f != 5;
+            }
+            e.sums = f == 5 ? c->red : nullptr;
+        }
+        return fft64_solve(c, d, cnt, s);
+    }
+
     // destination of the raw solution
     double* dst[6];
     for (int f = 0; f < 6; ++f) {
@@ -614,25 +636,20 @@ int solve_fields(lc3d_ctx* c, int which, const SolveInputs& in, const SolveOutpu
             }
             LC3D_TRY(mixed_stage(c, d, cnt, s));
         }
-    } else if (c->use_fft || c->p.precision == LC3D_PREC_FFT32) {
-        // four FFT row passes, each writing its output transposed; with the
-        // float32-transform precision the passes compute in float32 and the
-        // two intermediates (in the t1 / t2 planes) are float32
-        const bool f32 = c->p.precision == LC3D_PREC_FFT32;
-        const int types[4] = {f32 ? FFT_F64_F32 : FFT_F64, f32 ? FFT_F32 : FFT_F64, f32 ? FFT_F32 : FFT_F64,
-                              f32 ? FFT_F32_F64 : FFT_F64};
+    } else if (c->p.precision == LC3D_PREC_FFT32) {
+        // four FFT row passes, each writing its output transposed; the two
+        // intermediates (in the t1 / t2 planes) are float32
+        static const int types[4] = {FFT_F64_F32, FFT_F32, FFT_F32, FFT_F32_F64};
         // The fields' passes on several streams (forked after the right-hand
         // sides, joined before the finalize): with two, the E fields on the
         // solve's stream and the B fields on a second; with three, Ex Ey /
         // Bx By / Ez Bz. The groups' passes are independent, so the tail of
         // one group's pass, when only part of the SMs still work, is filled
-        // by the other groups' row groups. Measured at 641^2: float64 1802 ->
-        // 1864 xi-steps/s with two streams (1835 with three); float32
-        // transforms 2109 -> 2145 with two, 2176 with three. The per-launch
+        // by the other groups' row groups. Measured at 641^2: 2109 -> 2145
+        // xi-steps/s with two streams, 2176 with three. The per-launch
         // timing pass keeps one stream, and so do the steps of a batch graph
-        // (its branches overlap the simulations already: a 32-simulation scan
-        // measured 3772 aggregate xi-steps/s on one stream, 3600 on several).
-        const int nstreams = (c->prof_on || c->one_stream) ? 1 : f32 ? LC3D_FFT32_STREAMS : LC3D_FFT_STREAMS;
+        // (its branches overlap the simulations already).
+        const int nstreams = (c->prof_on || c->one_stream) ? 1 : LC3D_FFT32_STREAMS;
         auto group_of = [&](int f) {
             if (nstreams == 3) return f == 2 || f == 5 ? 2 : (f < 2 ? 0 : 1);
             if (nstreams == 2) return f < 3 ? 0 : 1;
@@ -654,15 +671,12 @@ int solve_fields(lc3d_ctx* c, int which, const SolveInputs& in, const SolveOutpu
                 const FieldGeom g = geom(c, f);
                 FftRowsDesc& e = d[cnt++];
                 memset(&e, 0, sizeof(e));
-                // the intermediates t1 / t2 at a row pitch of whole 32-byte
-                // sectors, so a CTA's transposed stores fill whole sectors
-                const int Np = fft_pitch(N, f32);
-                e.ld_in = stage == 0 ? N : Np;
-                e.ld_out = stage == 3 ? N : Np;
+                e.ld_in = N;
+                e.ld_out = N;
                 switch (stage) {
                     case 0: e.in = c->rhs[f] + g.off; e.rows = g.rows; e.type = g.type1; e.out = c->t1[f]; break;
                     case 1: e.in = c->t1[f]; e.rows = g.cols; e.type = g.type0; e.out = c->t2[f];
-                            e.lam = f32 ? static_cast<const void*>(lam32(c, f)) : g.Lam;
+                            e.lam = lam32(c, f);
                             e.ld_lam = g.ldLam; break;   // Lambda o Z as Z is written
                     case 2: e.in = c->t2[f]; e.rows = g.rows; e.type = g.type1; e.out = c->t1[f]; break;
                     default: e.in = c->t1[f]; e.rows = g.cols; e.type = g.type0; e.out = dst[f] + g.off;

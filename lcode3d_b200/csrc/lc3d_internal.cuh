@@ -176,36 +176,46 @@ struct SolveOutputs {
 int solve_fields(lc3d_ctx* ctx, int which, const SolveInputs& in,
                  const SolveOutputs& o, cudaStream_t s);
 
-// FFT row transforms (fields_fft.cu): rows of `in` (length N for DCT-I,
+// Float32 FFT row transforms (fields_fft.cu): rows of `in` (length N for DCT-I,
 // N - 2 for DST-I) are transformed and written transposed, out[k][r],
 // optionally multiplied element-wise by lam[k][r] as they are written.
-// Element types of a pass: the rows read, the arithmetic (and Lambda), the
-// rows written.
+// Element types of a pass: the rows read, the rows written (arithmetic and
+// Lambda are float).
 enum FftTypes {
-    FFT_F64 = 0,       // double -> double arithmetic -> double
-    FFT_F64_F32 = 1,   // double -> float -> float
-    FFT_F32 = 2,       // float -> float -> float
-    FFT_F32_F64 = 3,   // float -> float -> double
+    FFT_F64_F32 = 0,
+    FFT_F32 = 1,
+    FFT_F32_F64 = 2,
 };
 struct FftRowsDesc {
     const void* in;
     int ld_in, rows, type;                // type: 0 DCT-I, 1 DST-I
     void* out;
     int ld_out;
-    const void* lam;                      // in the arithmetic's type
+    const float* lam;
     int ld_lam;
     double* partial;                      // optional: per-CTA sums of the written values
 };
 int fft_init(lc3d_ctx* ctx);
-// Row pitch (elements) of the FFT passes' intermediate planes: float64 rows
-// padded to whole 32-byte sectors (N rounded up to a multiple of 4), so a
-// CTA's transposed 4-row stores fill whole sectors (transforms 0.319 ->
-// 0.317 ms per step at 641^2); float32 intermediates at N (padding them
-// measured slower: 0.235 -> 0.242).
-inline int fft_pitch(int N, bool f32 = false) { return f32 ? N : (N + 3) / 4 * 4; }
 int fft_cta_rows();                       // rows per CTA: partial sums per field = ceil(rows / this)
 int fft_rows(lc3d_ctx* ctx, const FftRowsDesc* desc, int count, int types, cudaStream_t s);
 int fft_plan(int P, int* rad);
+
+// Float64 FFT solves (fields_fft64.cu): the right-hand sides of `count` fields
+// through three launches to the fields, the step finalize included.
+struct Fft64Desc {
+    const double* rhs;                    // N x N plane; where an axis is DST-I its border is not read
+    int type0, type1;                     // axis-0 / axis-1 transform: 0 DCT-I, 1 DST-I
+    double *t1, *t2;                      // intermediates, N rows of fft64_pitch(N)
+    double* out;                          // N x N, zero border included; NULL: averages only
+    const double* prev;                   // with avg: the previous step's field
+    double* avg;                          // (out + prev) / 2, or NULL
+    int variant_a;                        // out = 2 F - prev
+    double* sums;                         // Bz: partial sums of the grid mean, subtracted from F
+};
+int fft64_init(lc3d_ctx* ctx);
+void fft64_free(lc3d_ctx* ctx);
+int fft64_pitch(int N);
+int fft64_solve(lc3d_ctx* ctx, const Fft64Desc* desc, int count, cudaStream_t s);
 
 // Mixed-precision transform stages (fields_mixed.cu): C = A B^T with one
 // operand a sliced fixed transform matrix (0 = S2, 1 = C) and the other the
@@ -280,8 +290,9 @@ struct lc3d_ctx {
     int red_blocks;
     int fft_ok, use_fft;                  // FFT transforms available / selected
     double* fft_tw;                       // FFT twiddles, P complex
-    int fft_grid[4];                      // persistent FFT grid per FftTypes instantiation
+    int fft_grid[3];                      // persistent FFT grid per FftTypes instantiation
     int fft_sms;                          // SMs of the device (the grid cap of lc3d_set_tiles)
+    void* fft64;                          // float64 FFT solves (fields_fft64.cu)
     void* mixed;                          // mixed-precision solver state (fields_mixed.cu)
     // launch accounting / profiling
     long long launches[LC3D_NSTAGES];

@@ -11,12 +11,11 @@
 //     c = hi * 2^-24 + lo * 2^-76 + (rounding below 2^-77),
 // which are summed with 64-bit integer adds; integer addition is associative,
 // so the sums do not depend on the order in which threads add them, and the
-// final conversion rounds once. Each CTA owns a tile of 8 (or 4, 16) fine
+// final conversion rounds once. Each CTA owns a tile of 12 (or 4, 8, 16) fine
 // lattice rows x 32 columns and accumulates into a shared-memory window
 // placed on the bounding box of its particles' cells (float64 sums in a
-// fixed order); particles whose stencil falls outside the window (strongly
-// displaced plasma) add straight to the global accumulators. The window is
-// then flushed with 64-bit integer reductions into global memory, and a
+// fixed order); particles outside the window (strongly displaced plasma) add
+// straight to the global accumulators. The window is then flushed with 64-bit integer reductions into global memory, and a
 // finalize pass converts to float64, adds the ion background and clears the
 // accumulators for the next call.
 
@@ -263,6 +262,54 @@ __device__ __forceinline__ void particle_values(FineParticle& p, double m, doubl
     p.djz = pz * dro_g;
 }
 
+// particle_values without branches, so that the chains of a thread's
+// particles overlap (the library's square root and division each end a block
+// of instructions with a test for their slow path: phase 1 of the deposition
+// took 43 of 83 us with them). Goldschmidt's iteration for sqrt(S) and
+// 1 / (2 sqrt(S)), Newton's for the reciprocal of the divisor, from the
+// hardware's approximations; each result is corrected by its exact residual
+// (Markstein), as particle_values' are. Returns false where S is not well
+// inside the range of normal numbers: the caller takes particle_values.
+__device__ __forceinline__ bool particle_values_fast(FineParticle& p, double m, double q, double px, double py,
+                                                     double pz) {
+    const double S = m * m + px * px + py * py + pz * pz;
+    double y, r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(S));
+    double g = S * y, h = .5 * y;
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+        const double e = fma(-g, h, .5);
+        g = fma(g, e, g);
+        h = fma(h, e, h);
+    }
+    g = fma(fma(-g, g, S), h, g);
+    double inv = h + h;
+    inv = fma(inv, fma(-g, inv, 1.0), inv);
+    const double d = 1 - div_h(pz, g, inv);
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+#pragma unroll
+    for (int it = 0; it < 2; ++it) r = fma(r, fma(-d, r, 1.0), r);
+    p.dro = div_h(q, d, r);
+    const double dro_g = div_h(p.dro, g, inv);
+    p.djx = px * dro_g;
+    p.djy = py * dro_g;
+    p.djz = pz * dro_g;
+    return S > 0x1p-900 && S < 0x1p900;
+}
+
+// The cell of one coordinate and the offset from its centre (tsc_cell): the
+// same floor, through the rounding of x_h + 1.5 2^52, whose low word is the
+// integer.
+__device__ __forceinline__ int tsc_cell_1(double x, int N, double h, double inv_h, double& xl) {
+    constexpr double M = 0x1.8p52;
+    const double x_h = div_h(x, h, inv_h) + .5;
+    const double t = x_h + M;
+    const bool up = t - M > x_h;
+    const double f = up ? (t - M) - 1.0 : t - M;
+    xl = x_h - f - .5;
+    return fabs(x_h) < 1.0e6 ? __double2loint(t) - (up ? 1 : 0) + N / 2 : -1;
+}
+
 __device__ __forceinline__ FineParticle fine_particle(const DepositArgs& a, int fi, int fj) {
     const double ipi = a.inf_prev[fi], ini = a.inf_next[fi];
     const double ipj = a.inf_prev[fj], inj = a.inf_next[fj];
@@ -305,76 +352,71 @@ __device__ __forceinline__ void fx_add(unsigned long long* hi_plane, unsigned lo
 }
 
 // ---------------------------------------------------------------------------
-// Deposition kernel. A CTA of TI warps deposits TI fine-lattice rows x 32
-// columns; one thread per fine particle, then one per (2 x 2 block, field).
-//  1. Coarse->fine mix in two separable passes (the equivalent formula noted
-//     beside the reference's make_plasma, lcode.py:554-556). Each warp holds
-//     one fine row fi of the tile; it first mixes the two coarse rows of fi,
+// Deposition kernel. A CTA deposits a tile of TI fine-lattice rows x 32
+// columns, three rows per warp.
+//  1. Three fine particles per thread, one per row of its warp. Coarse->fine
+//     mix in two separable passes (the equivalent formula noted beside the
+//     reference's make_plasma, lcode.py:554-556): the warp first mixes the two
+//     coarse rows of each fine row fi,
 //         R[c] = inf_prev[fi] Q[prev_i][c] + inf_next[fi] Q[next_i][c],
-//     for every coarse column c its 32 fine columns use (7 quantities, a
-//     warp-private shared-memory table), and each lane then mixes two
-//     entries, Q = inf_prev[fj] R[prev_j] + inf_next[fj] R[next_j]: 14
-//     float64 operations and 8 shared loads per particle, no CTA barrier. A
-//     tile whose columns span more than DEP2_CMAX coarse columns (other
-//     coarseness / fineness settings, or arbitrary virt_params) mixes per
-//     particle from global memory (fine_particle). Then the deposit values
-//     (lcode.py:651-655) and the TSC cell, staged in shared memory; the CTA's
-//     bounding box of cells places the window.
-//  2. One thread per (2 x 2 block of fine particles, field). If the block's
-//     centre cells span at most 2 x 2 cells -- neighbouring fine particles
-//     are interpolated from the same coarse particles and move together --
-//     its four TSC stencils are summed in a fixed order into a register
-//     patch: 3 x 3 when all four lie in one cell, else 4 x 4. Tiles start
-//     `a.fine_off` fine particles before the lattice origin: with an even
-//     fineness the lattice has two particles per cell and axis and the fine
-//     index pairs (odd, even) share a cell, so with an offset of 1 every
-//     block of an undisturbed lattice lies in one cell (9 window entries and
-//     36 products per field instead of 16 and 64). Blocks claim their patch's
-//     corner cell (atomicMax of the block index: the winner does not depend
-//     on timing); winners add their patches to the window in 9 or 16
-//     barrier-separated steps, one patch entry per step, so in each step
-//     every window cell has at most one writer and its summation order is
-//     fixed. Losing blocks (two on one corner) and blocks that span more
-//     cells or leave the window add their contributions straight to the
-//     global accumulators through the exact split.
+//     for the coarse columns c its lanes use (7 quantities, a warp-private
+//     table in shared memory); each lane then mixes two entries,
+//     Q = inf_prev[fj] R[prev_j] + inf_next[fj] R[next_j]. A tile whose
+//     columns span more than DEP_CMAX coarse columns (other coarseness /
+//     fineness settings, or arbitrary virt_params) mixes per particle from
+//     global memory (fine_particle). Then the deposit values
+//     (lcode.py:651-655) and the TSC cell; cell offsets and values are staged
+//     in shared memory.
+//  2. One thread per cell. Every particle sets its bit in its cell's masks
+//     (one word per fine row, one bit per column), so a cell's thread meets
+//     its particles in the order of the lattice, whatever the timing. It sums
+//     their stencils, all four fields, into a 3 x 3 patch in registers: the
+//     weights of a particle are computed once, and a patch never spans more
+//     than one cell, however the lattice has moved against the grid. The
+//     patches are added to a float64 window in nine barrier-separated steps,
+//     one patch entry a step: no two threads write one cell in a step.
 //  3. Each touched window cell is split once into fixed point and added to
-//     the global accumulators.
+//     the global accumulators. A tile whose cells are too many for one window
+//     (rarefied plasma) takes up to four, one strip of rows after the other;
+//     particles outside all of them add straight to the accumulators.
+//
+// Tiles start `a.fine_off` fine particles before the lattice origin: with an
+// even fineness the fine index pairs (odd, even) of an undisturbed lattice
+// share a cell, so no row or column of cells is split between tiles.
+//
+// Bound by instruction issue and latency, at 16 warps per SM (the patch's 72
+// registers): 641^2, plasma displaced by several cells, 33.4 M warp
+// instructions of which 10.9 M float64, issue 50 %, 62 us a launch. Summing
+// 2 x 2 blocks of the lattice per (block, field) instead, with their weights
+// once per field and 4 x 4 patches wherever a block straddles cells, took 45 M
+// and 88 us. Per phase (us): lattice and row tables 13, particles 14, masks 5,
+// sums over cells 18, window steps 7, flush 6. Five CTAs per SM (96
+// registers, spills) measured 71 against 67, cells listed fullest first 67
+// against 66.
 // ---------------------------------------------------------------------------
-#ifndef LC3D_DEP2_CLOCKS
-#define LC3D_DEP2_CLOCKS 0
-#endif
-constexpr int DEP2_CMAX = 16;               // coarse columns one row table holds
-constexpr int DEP2_WC = 32;                 // window columns (cells); rows: 2 per fine row of the tile
+constexpr int DEP_TW = 32;                  // fine columns of a tile, one per lane
+constexpr int DEP_RPW = 3;                  // fine rows per warp
+constexpr int DEP_CMAX = 16;                // coarse columns the row tables hold
+constexpr int DEP_CELLS = 256;              // cells with particles in a window
+constexpr int DEP_SIDE = 32;                // ... their rows or columns at most
+constexpr int DEP_STRIPS = 4;               // windows of a tile, one after the other (rarefied plasma)
+constexpr int DEP_WIN = 352;                // window cells, (rows + 2) (columns + 2) <= 340
 
-// Dynamic shared memory of a tile of `ti` fine rows x 32 columns.
-constexpr size_t dep2_smem(int ti) {
-    return (size_t)ti * DEP2_CMAX * 8 * sizeof(double)              // row tables
-           + (size_t)ti * 32 * (6 * sizeof(double) + sizeof(int))   // staging
-           + (size_t)4 * (2 * ti * DEP2_WC) * sizeof(double)        // window, 4 fields
-           + (size_t)(2 * ti * DEP2_WC) * sizeof(int);               // anchor claims
+// Threads of a tile of `ti` rows. 12 rows: 384 particles on 128 threads, and
+// at most 7 x 17 cells of an undisturbed lattice, one round of the threads (us
+// per xi step with 12 / 4 / 8 / 16 rows: 641^2 367 / 419 / 375 / 402, 321^2
+// 132 / 160 / 137 / 138, 161^2 86.5 / 86.1 / 83.2 / 84.3).
+__host__ __device__ constexpr int dep_threads(int ti) { return (ti + DEP_RPW - 1) / DEP_RPW * 32; }
+
+template <int TI>
+__host__ __device__ constexpr size_t dep_table_words() {   // double2 words: the row tables, then the window
+    constexpr size_t table = (size_t)TI * DEP_CMAX * 4, win = 2 * DEP_WIN;
+    return table > win ? table : win;
 }
-
-#if LC3D_DEP2_CLOCKS
-constexpr int DEP2_NCLK = 6;
-__device__ long long g_dep2_clocks[16384][DEP2_NCLK];
-#define DEP2_CLK(k)                                                                      \
-    do {                                                                                 \
-        if (threadIdx.x == 0) {                                                          \
-            const int cta = blockIdx.y * gridDim.x + blockIdx.x;                         \
-            if (cta < 16384) g_dep2_clocks[cta][k] = clock64() - clk0;                   \
-        }                                                                                \
-    } while (0)
-#else
-#define DEP2_CLK(k) do { } while (0)
-#endif
-
-// TSC weights of staged particle k from its staged cell offsets (xl at
-// s_pos[k], yl at s_pos[threads + k]). Staging the six weights instead
-// measured slower (shared-memory traffic against 12 float64 operations).
-__device__ __forceinline__ void staged_weights(const double* s_pos, int threads, int k, double& wxM, double& wx0,
-                                               double& wxP, double& wyM, double& wy0, double& wyP) {
-    tsc_axis(s_pos[k], wxM, wx0, wxP);
-    tsc_axis(s_pos[threads + k], wyM, wy0, wyP);
+template <int TI>
+constexpr size_t dep_smem() {
+    return ((size_t)TI * DEP_TW * 3 + dep_table_words<TI>()) * sizeof(double2)   // (xl, yl), (ro, jx), (jy, jz); table
+           + (TI + 1) * DEP_CELLS * sizeof(unsigned);                            // masks, rows in use
 }
 
 // Two of the seven coarse quantities of coarse particle k as a pair: h = 0
@@ -389,272 +431,280 @@ __device__ __forceinline__ double2 coarse_pair(const DepositArgs& a, int k, int 
     }
 }
 
-// TI fine rows x 32 fine columns per CTA, one warp per row (TI = 4, 8, 16:
-// 8, 4 or 2 resident CTAs per SM at 64 registers).
 template <int TI>
 __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, int tile_y) {
-    constexpr int DEP2_TI = TI;
-    constexpr int DEP2_THREADS = DEP2_TI * 32;
-    constexpr int DEP2_BLOCKS = DEP2_THREADS / 4;
-    constexpr int DEP2_WR = 2 * DEP2_TI;   // window rows (cells)
-    constexpr int DEP2_WIN = DEP2_WR * DEP2_WC;
-    static_assert(DEP2_TI % 2 == 0 && DEP2_TI <= 32, "2 x 2 blocks, at most 32 warps");
-#if LC3D_DEP2_CLOCKS
-    const long long clk0 = clock64();
-#endif
-    extern __shared__ double smem_f64[];
-    double2* s_R = reinterpret_cast<double2*>(smem_f64);                 // [DEP2_TI][DEP2_CMAX][4]
-    double* s_pos = smem_f64 + DEP2_TI * DEP2_CMAX * 8;                  // cell offsets xl, yl: [2][DEP2_THREADS]
-    double* s_xl = s_pos;
-    double* s_yl = s_xl + DEP2_THREADS;
-    double* s_v = s_yl + DEP2_THREADS;                                   // [4][DEP2_THREADS]
-    double* s_win = s_v + 4 * DEP2_THREADS;                              // [4][DEP2_WIN]
-    int* s_claim = reinterpret_cast<int*>(s_win + 4 * DEP2_WIN);         // [DEP2_WIN]
-    int* s_cell = s_claim + DEP2_WIN;                                    // [DEP2_THREADS]: i << 16 | j, or -1
+    constexpr int T = dep_threads(TI), P = TI * DEP_TW;
+    static_assert(TI <= 32, "masks of 32 bits");
+    extern __shared__ __align__(16) double smem_f64[];
+    double2* s_pos = reinterpret_cast<double2*>(smem_f64);               // [P] cell offsets
+    double2* s_v01 = s_pos + P;                                          // [P] ro, jx
+    double2* s_v23 = s_v01 + P;                                          // [P] jy, jz
+    double2* s_R = s_v23 + P;                                            // [TI][DEP_CMAX][4]; then the window
+    double* s_win = reinterpret_cast<double*>(s_R);                      // [4][DEP_WIN]
+    unsigned* s_mask = reinterpret_cast<unsigned*>(s_R + dep_table_words<TI>());   // [TI][DEP_CELLS]
+    unsigned* s_rows = s_mask + TI * DEP_CELLS;                          // [DEP_CELLS]
     __shared__ int s_bb[4];                                              // imin imax jmin jmax
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int t = threadIdx.x, lane = t & 31, row0 = (t >> 5) * DEP_RPW;
     if (t == 0) {
         s_bb[0] = s_bb[2] = 1 << 30;
         s_bb[1] = s_bb[3] = -(1 << 30);
     }
-    for (int w = t; w < 4 * DEP2_WIN; w += DEP2_THREADS) s_win[w] = 0.0;
-    for (int w = t; w < DEP2_WIN; w += DEP2_THREADS) s_claim[w] = -1;
+    {
+        uint4* z = reinterpret_cast<uint4*>(s_mask);
+        for (int w = t; w < (TI + 1) * DEP_CELLS / 4; w += T) z[w] = make_uint4(0u, 0u, 0u, 0u);
+    }
     const int N = a.N;
     const size_t NN = a.plane;
     pdl_wait();   // global memory from here on
-    DEP2_CLK(0);
 
-    // ---- phase 1: one fine particle per thread; warp = fine row ----
+    // ---- phase 1 ----
+    const int fi0 = tile_y * TI - a.fine_off + row0, fj = tile_x * DEP_TW - a.fine_off + lane;
+    const bool col_ok = fj >= 0 && fj < a.Nf;
+    int pi[DEP_RPW], ni[DEP_RPW], pj = 0, nj = 0;
+    double ipi[DEP_RPW], ini[DEP_RPW], fgi[DEP_RPW], ipj = 0, inj = 0, fgj = 0;
+    bool row_ok[DEP_RPW];
+#pragma unroll
+    for (int u = 0; u < DEP_RPW; ++u) {
+        const int fi = fi0 + u;
+        row_ok[u] = row0 + u < TI && fi >= 0 && fi < a.Nf;
+        pi[u] = ni[u] = 0;
+        ipi[u] = ini[u] = fgi[u] = 0;
+        if (row_ok[u]) {
+            pi[u] = a.idx_prev[fi];
+            ni[u] = a.idx_next[fi];
+            ipi[u] = a.inf_prev[fi];
+            ini[u] = a.inf_next[fi];
+            fgi[u] = a.fine_grid[fi];
+        }
+    }
+    if (col_ok) {
+        pj = a.idx_prev[fj];
+        nj = a.idx_next[fj];
+        ipj = a.inf_prev[fj];
+        inj = a.inf_next[fj];
+        fgj = a.fine_grid[fj];
+    }
+    const bool col_idx = pj >= 0 && pj < a.Nc && nj >= 0 && nj < a.Nc;
+    // the coarse columns of the tile (the same in every warp)
+    const int c0 = __reduce_min_sync(0xffffffffu, col_ok ? (col_idx ? min(pj, nj) : -(1 << 30)) : 1 << 30);
+    const int c1 = __reduce_max_sync(0xffffffffu, col_ok ? (col_idx ? max(pj, nj) : 1 << 30) : -(1 << 30));
+    const int nc = c1 - c0 + 1;
+    const bool staged = c0 >= 0 && nc >= 1 && nc <= DEP_CMAX;
+    bool ok[DEP_RPW];
+#pragma unroll
+    for (int u = 0; u < DEP_RPW; ++u) {
+        const bool idx = pi[u] >= 0 && pi[u] < a.Nc && ni[u] >= 0 && ni[u] < a.Nc;
+        if (row_ok[u] && col_ok && !(idx && col_idx)) atomicOr(a.err, LC3D_FLAG_WINDOW);
+        if (!idx) pi[u] = ni[u] = 0;   // nobody uses that row of the table
+        ok[u] = row_ok[u] && col_ok && idx && col_idx;
+    }
+    double2* R = s_R + row0 * DEP_CMAX * 4;
+    if (staged) {
+        for (int it = lane; it < nc * 4; it += 32) {
+            const int jc = it >> 2, h = it & 3;
+            double2 qp[DEP_RPW], qn[DEP_RPW];
+#pragma unroll
+            for (int u = 0; u < DEP_RPW; ++u) {
+                if (row0 + u >= TI) continue;
+                qp[u] = coarse_pair(a, pi[u] * a.Nc + c0 + jc, h);
+                qn[u] = coarse_pair(a, ni[u] * a.Nc + c0 + jc, h);
+            }
+#pragma unroll
+            for (int u = 0; u < DEP_RPW; ++u) {
+                if (row0 + u >= TI) continue;
+                R[u * DEP_CMAX * 4 + it] = make_double2(ipi[u] * qp[u].x + ini[u] * qn[u].x,
+                                                        ipi[u] * qp[u].y + ini[u] * qn[u].y);
+            }
+        }
+    }
+    __syncwarp();
+    int cell[DEP_RPW];   // i << 16 | j, or -1
     {
-        const int fi = tile_y * DEP2_TI + warp - a.fine_off;
-        const int fj = tile_x * 32 + lane - a.fine_off;
-        const bool row_ok = fi >= 0 && fi < a.Nf, col_ok = fj >= 0 && fj < a.Nf;
-        // every input of the particle first (independent loads), then the
-        // coarse rows of the row table
-        int pi = 0, ni = 0, pj = 0, nj = 0;
-        double ipi = 0, ini = 0, fgi = 0, ipj = 0, inj = 0, fgj = 0;
-        if (row_ok) {
-            pi = a.idx_prev[fi];
-            ni = a.idx_next[fi];
-            ipi = a.inf_prev[fi];
-            ini = a.inf_next[fi];
-            fgi = a.fine_grid[fi];
-        }
-        if (col_ok) {
-            pj = a.idx_prev[fj];
-            nj = a.idx_next[fj];
-            ipj = a.inf_prev[fj];
-            inj = a.inf_next[fj];
-            fgj = a.fine_grid[fj];
-        }
-        const bool row_idx = pi >= 0 && pi < a.Nc && ni >= 0 && ni < a.Nc;
-        const bool col_idx = pj >= 0 && pj < a.Nc && nj >= 0 && nj < a.Nc;
-        // the coarse columns of the tile (the same in every warp)
-        const int c0 = __reduce_min_sync(0xffffffffu, col_ok ? (col_idx ? min(pj, nj) : -(1 << 30)) : 1 << 30);
-        const int c1 = __reduce_max_sync(0xffffffffu, col_ok ? (col_idx ? max(pj, nj) : 1 << 30) : -(1 << 30));
-        const int nc = c1 - c0 + 1;
-        const bool staged = c0 >= 0 && nc >= 1 && nc <= DEP2_CMAX;
-        double2* R = s_R + warp * DEP2_CMAX * 4;
-        if (staged && row_ok && row_idx) {
-            for (int it = lane; it < nc * 4; it += 32) {
-                const int jc = it >> 2, h = it & 3;
-                const double2 qp = coarse_pair(a, pi * a.Nc + c0 + jc, h);
-                const double2 qn = coarse_pair(a, ni * a.Nc + c0 + jc, h);
-                R[it] = make_double2(ipi * qp.x + ini * qn.x, ipi * qp.y + ini * qn.y);
-            }
-        }
-        __syncwarp();
-        int cell = -1, i = 1 << 30, j = 1 << 30;
-        if (row_ok && col_ok) {
-            if (!(row_idx && col_idx)) {
-                atomicOr(a.err, LC3D_FLAG_WINDOW);
-            } else {
-                FineParticle f;
-                if (staged) {
-                    const double2* Rp = R + (pj - c0) * 4;
-                    const double2* Rn = R + (nj - c0) * 4;
-                    double2 q[4];
+        const int op = (staged && col_ok ? pj - c0 : 0) * 4, on = (staged && col_ok ? nj - c0 : 0) * 4;
+        FineParticle f[DEP_RPW];
+        bool slow = !staged;
+        double q[DEP_RPW][5];
+        if (staged) {
 #pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        const double2 rp = Rp[h], rn = Rn[h];
-                        q[h] = make_double2(ipj * rp.x + inj * rn.x, ipj * rp.y + inj * rn.y);
-                    }
-                    f.x = fgi + q[0].x;
-                    f.y = fgj + q[0].y;
-                    particle_values(f, a.sf * q[1].x, a.sf * q[1].y, a.sf * q[2].x, a.sf * q[2].y,
-                                    a.sf * q[3].x);
-                } else {
-                    f = fine_particle(a, fi, fj);
+            for (int u = 0; u < DEP_RPW; ++u) {
+                const double2* Ru = R + (row0 + u < TI ? u : 0) * DEP_CMAX * 4;
+                double2 w[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const double2 rp = Ru[op + h], rn = Ru[on + h];
+                    w[h] = make_double2(ipj * rp.x + inj * rn.x, ipj * rp.y + inj * rn.y);
                 }
-                double xl, yl;
-                tsc_cell(f.x, f.y, N, a.h, a.inv_h, i, j, xl, yl);
-                const double vmax = fmax(fmax(fabs(f.dro), fabs(f.djx)), fmax(fabs(f.djy), fabs(f.djz)));
-                if (!(i >= 1 && i <= N - 2 && j >= 1 && j <= N - 2)) {
-                    atomicOr(a.err, LC3D_FLAG_WINDOW);
-                } else if (!(vmax < FX_MAX)) {   // also catches NaN
-                    atomicOr(a.err, LC3D_FLAG_NONFINITE);
-                } else {
-                    cell = (i << 16) | j;
-                }
-                s_xl[t] = xl;
-                s_yl[t] = yl;
-                s_v[t] = f.dro;
-                s_v[DEP2_THREADS + t] = f.djx;
-                s_v[2 * DEP2_THREADS + t] = f.djy;
-                s_v[3 * DEP2_THREADS + t] = f.djz;
+                f[u].x = fgi[u] + w[0].x;
+                f[u].y = fgj + w[0].y;
+                q[u][0] = a.sf * w[1].x;
+                q[u][1] = a.sf * w[1].y;
+                q[u][2] = a.sf * w[2].x;
+                q[u][3] = a.sf * w[2].y;
+                q[u][4] = a.sf * w[3].x;
             }
+#pragma unroll
+            for (int u = 0; u < DEP_RPW; ++u)
+                if (!particle_values_fast(f[u], q[u][0], q[u][1], q[u][2], q[u][3], q[u][4]) && ok[u]) slow = true;
         }
-        s_cell[t] = cell;
-        // warp bounding box of the cells (one redux instruction each)
-        const int imin = __reduce_min_sync(0xffffffffu, cell >= 0 ? i : 1 << 30);
-        const int imax = __reduce_max_sync(0xffffffffu, cell >= 0 ? i : -(1 << 30));
-        const int jmin = __reduce_min_sync(0xffffffffu, cell >= 0 ? j : 1 << 30);
-        const int jmax = __reduce_max_sync(0xffffffffu, cell >= 0 ? j : -(1 << 30));
-        __syncthreads();   // s_bb initialised, window and claims cleared
-        if (lane == 0 && imin <= imax) {
-            atomicMin(&s_bb[0], imin);
-            atomicMax(&s_bb[1], imax);
-            atomicMin(&s_bb[2], jmin);
-            atomicMax(&s_bb[3], jmax);
-        }
-    }
-    __syncthreads();
-    DEP2_CLK(1);
-
-    // ---- phase 2: one (2 x 2 block, field) per thread ----
-    const int f = t / DEP2_BLOCKS, blk = t % DEP2_BLOCKS;
-    const int p0 = (blk >> 4) * 64 + (blk & 15) * 2;   // top-left particle of the block
-    const int pidx[4] = {p0, p0 + 1, p0 + 32, p0 + 33};
-    int ci[4], cj[4];
-    bool ok[4];
-    int i0 = 1 << 30, i1 = -(1 << 30), j0 = 1 << 30, j1 = -(1 << 30);
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        const int c = s_cell[pidx[p]];
-        ok[p] = c >= 0;
-        ci[p] = c >> 16;
-        cj[p] = c & 0xffff;
-        if (ok[p]) {
-            i0 = min(i0, ci[p]);
-            i1 = max(i1, ci[p]);
-            j0 = min(j0, cj[p]);
-            j1 = max(j1, cj[p]);
-        }
-    }
-    const int oi = s_bb[0] - 1, oj = s_bb[2] - 1;   // window origin (cells)
-    const bool patch = i0 <= i1 && i1 - i0 <= 1 && j1 - j0 <= 1 && i0 + 2 - oi < DEP2_WR && j0 + 2 - oj < DEP2_WC;
-    const bool one = patch && i1 == i0 && j1 == j0;   // all four in one cell: a 3 x 3 patch
-    const int ar = i0 - 1, ac = j0 - 1;             // the patch's corner cell
-    const int r0 = ar - oi, c0w = ac - oj;          // ... in window coordinates
-    if (patch && f == 0) atomicMax(&s_claim[r0 * DEP2_WC + c0w], blk);
-    __syncthreads();
-    const bool winner = patch && s_claim[r0 * DEP2_WC + c0w] == blk;
-    unsigned long long* ghi = a.acc + (2 * f) * NN;
-    unsigned long long* glo = ghi + NN;
-    const double* vf = s_v + f * DEP2_THREADS;
-    double acc[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) acc[k] = 0.0;
-    if (one) {
-        // the four stencils on the same 3 x 3 cells: entry (r, c) of the
-        // patch is acc[r * 4 + c], r, c < 3
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            if (!ok[p]) continue;
-            double wx[3], wy[3];
-            staged_weights(s_pos, DEP2_THREADS, pidx[p], wx[0], wx[1], wx[2], wy[0], wy[1], wy[2]);
-            const double v = vf[pidx[p]];
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                const double vx = v * wx[r];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) acc[r * 4 + c] = fma(vx, wy[c], acc[r * 4 + c]);
-            }
-        }
-    } else if (patch) {
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            if (!ok[p]) continue;
-            double wxM, wx0, wxP, wyM, wy0, wyP;
-            staged_weights(s_pos, DEP2_THREADS, pidx[p], wxM, wx0, wxP, wyM, wy0, wyP);
-            const bool si = ci[p] != i0, sj = cj[p] != j0;
-            const double wx4[4] = {si ? 0.0 : wxM, si ? wxM : wx0, si ? wx0 : wxP, si ? wxP : 0.0};
-            const double wy4[4] = {sj ? 0.0 : wyM, sj ? wyM : wy0, sj ? wy0 : wyP, sj ? wyP : 0.0};
-            const double v = vf[pidx[p]];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const double vx = v * wx4[r];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r * 4 + c] = fma(vx, wy4[c], acc[r * 4 + c]);
-            }
-        }
-    } else {
+        if (slow) {
 #pragma unroll 1
-        for (int p = 0; p < 4; ++p) {
-            const int c = s_cell[pidx[p]];
-            if (c < 0) continue;
-            const int pi = c >> 16, pj = c & 0xffff;
-            double wx[3], wy[3];
-            staged_weights(s_pos, DEP2_THREADS, pidx[p], wx[0], wx[1], wx[2], wy[0], wy[1], wy[2]);
-            const double v = vf[pidx[p]];
+            for (int u = 0; u < DEP_RPW; ++u)
+                if (u == 0 ? ok[0] : u == 1 ? ok[1] : ok[2]) {
+                    const FineParticle g = fine_particle(a, fi0 + u, fj);
 #pragma unroll
-            for (int di = 0; di < 3; ++di)
-#pragma unroll
-                for (int dj = 0; dj < 3; ++dj)
-                    fx_add(ghi, glo, (size_t)(pi + di - 1) * N + (pj + dj - 1), v * (wx[di] * wy[dj]));
-        }
-    }
-    if (patch && !winner) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (acc[r * 4 + c] != 0.0) fx_add(ghi, glo, (size_t)(ar + r) * N + (ac + c), acc[r * 4 + c]);
-    }
-    DEP2_CLK(2);
-    // winners add their patches, one entry per barrier-separated step; a
-    // CTA whose blocks all lie in single cells needs only the 9 entries of
-    // a 3 x 3 patch
-    double* fw = s_win + f * DEP2_WIN + (winner ? r0 * DEP2_WC + c0w : 0);
-    if (__syncthreads_or(patch && !one)) {   // uniform over the CTA
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            if (winner && acc[k] != 0.0) fw[(k >> 2) * DEP2_WC + (k & 3)] += acc[k];
-            __syncthreads();
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < 9; ++e) {
-            const int k = (e / 3) * 4 + e % 3;
-            if (winner && acc[k] != 0.0) fw[(k >> 2) * DEP2_WC + (k & 3)] += acc[k];
-            __syncthreads();
-        }
-    }
-    DEP2_CLK(3);
-
-    // ---- phase 3: split each touched window cell once, add to global ----
-    if (s_bb[0] <= s_bb[1]) {
-        // lane = window column (the window is 32 cells wide), warps step over
-        // the rows of each field: consecutive lanes add to consecutive cells
-        const int ni = min(s_bb[1] + 2 - oi, DEP2_WR), nj = min(s_bb[3] + 2 - oj, DEP2_WC);
-        static_assert(DEP2_WC == 32, "one lane per window column");
-        if (lane < nj) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                unsigned long long* hi = a.acc + (2 * q) * NN;
-                for (int r = warp; r < ni; r += DEP2_TI) {
-                    const double v = s_win[q * DEP2_WIN + r * DEP2_WC + lane];
-                    if (v != 0.0) fx_add(hi, hi + NN, (size_t)(oi + r) * N + (oj + lane), v);
+                    for (int k = 0; k < DEP_RPW; ++k)
+                        if (k == u) f[k] = g;
                 }
+        }
+#pragma unroll
+        for (int u = 0; u < DEP_RPW; ++u) {
+            double xl, yl;
+            const int i = tsc_cell_1(f[u].x, N, a.h, a.inv_h, xl), j = tsc_cell_1(f[u].y, N, a.h, a.inv_h, yl);
+            const bool in = i >= 1 && i <= N - 2 && j >= 1 && j <= N - 2;
+            // also false for NaN
+            const bool fin = fabs(f[u].dro) < FX_MAX && fabs(f[u].djx) < FX_MAX && fabs(f[u].djy) < FX_MAX &&
+                             fabs(f[u].djz) < FX_MAX;
+            if (ok[u] && !(in && fin)) atomicOr(a.err, in ? LC3D_FLAG_NONFINITE : LC3D_FLAG_WINDOW);
+            cell[u] = ok[u] && in && fin ? (i << 16) | j : -1;
+            if (cell[u] >= 0) {
+                const int k = (row0 + u) * DEP_TW + lane;
+                s_pos[k] = make_double2(xl, yl);
+                s_v01[k] = make_double2(f[u].dro, f[u].djx);
+                s_v23[k] = make_double2(f[u].djy, f[u].djz);
             }
         }
     }
-    DEP2_CLK(4);
+    int imin = 1 << 30, imax = -(1 << 30), jmin = 1 << 30, jmax = -(1 << 30);
+#pragma unroll
+    for (int u = 0; u < DEP_RPW; ++u) {
+        if (cell[u] < 0) continue;
+        const int i = cell[u] >> 16, j = cell[u] & 0xffff;
+        imin = min(imin, i);
+        imax = max(imax, i);
+        jmin = min(jmin, j);
+        jmax = max(jmax, j);
+    }
+    imin = __reduce_min_sync(0xffffffffu, imin);
+    imax = __reduce_max_sync(0xffffffffu, imax);
+    jmin = __reduce_min_sync(0xffffffffu, jmin);
+    jmax = __reduce_max_sync(0xffffffffu, jmax);
+    if (lane == 0 && imin <= imax) {
+        atomicMin(&s_bb[0], imin);
+        atomicMax(&s_bb[1], imax);
+        atomicMin(&s_bb[2], jmin);
+        atomicMax(&s_bb[3], jmax);
+    }
+    __syncthreads();   // the bounding box; the row tables are done with
+    if (s_bb[0] > s_bb[1]) return;   // no particle (uniform)
+    const int oj = s_bb[2], mj = min(s_bb[3] - oj + 1, DEP_SIDE);   // the first column of cells with particles, columns
+    const int strip_rows = min(DEP_SIDE, DEP_CELLS / mj), wj = mj + 2;
+    const int strips = min((s_bb[1] - s_bb[0]) / strip_rows + 1, DEP_STRIPS);
+    for (int strip = 0; strip < strips; ++strip) {
+        // this window's cells with particles: mi rows from oi, mj columns from
+        // oj; the window holds one cell more on each side
+        const int oi = s_bb[0] + strip * strip_rows, mi = min(s_bb[1] - oi + 1, strip_rows);
+        const int nwin = (mi + 2) * wj, ncell = mi * mj;
+        for (int w = t; w < nwin; w += T)
+#pragma unroll
+            for (int f = 0; f < 4; ++f) s_win[f * DEP_WIN + w] = 0.0;
+        if (strip) {   // the first window's masks were cleared above
+            uint4* z = reinterpret_cast<uint4*>(s_mask);
+            for (int w = t; w < (TI + 1) * DEP_CELLS / 4; w += T) z[w] = make_uint4(0u, 0u, 0u, 0u);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int u = 0; u < DEP_RPW; ++u) {
+            if (cell[u] < 0) continue;
+            const int row = row0 + u, i = (cell[u] >> 16) - oi, j = (cell[u] & 0xffff) - oj;
+            if (i >= 0 && i < mi && j < mj) {
+                const int c = i * mj + j;
+                atomicOr(&s_mask[row * DEP_CELLS + c], 1u << lane);
+                atomicOr(&s_rows[c], 1u << row);
+            } else if (strip == 0 && (j >= mj || i >= strips * strip_rows)) {   // in no window
+                const int k = row * DEP_TW + lane;
+                unsigned long long* g = a.acc + (size_t)(oi + i - 1) * N + (oj + j - 1);
+                double wx[3], wy[3];
+                tsc_axis(s_pos[k].x, wx[0], wx[1], wx[2]);
+                tsc_axis(s_pos[k].y, wy[0], wy[1], wy[2]);
+#pragma unroll 1
+                for (int f = 0; f < 4; ++f) {
+                    const double v = f == 0 ? s_v01[k].x : f == 1 ? s_v01[k].y : f == 2 ? s_v23[k].x : s_v23[k].y;
+#pragma unroll
+                    for (int e = 0; e < 9; ++e)
+                        fx_add(g + 2 * f * NN, g + (2 * f + 1) * NN, (size_t)(e / 3) * N + e % 3, v * (wx[e / 3] * wy[e % 3]));
+                }
+            }
+        }
+        __syncthreads();   // masks complete, window cleared
+
+        // ---- phase 2: one cell per thread ----
+        const float inv_mj = 1.0f / (float)mj;
+        for (int r0 = 0; r0 < ncell; r0 += T) {
+            const int c = r0 + t;
+            unsigned rows = c < ncell ? s_rows[c] : 0u, m = 0;
+            const bool any = rows != 0;
+            const unsigned* mk = s_mask + c;
+            int base = 0;
+            double acc[4][9];
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+#pragma unroll
+                for (int e = 0; e < 9; ++e) acc[f][e] = 0.0;
+            while (rows | m) {
+                if (!m) {
+                    const int r = __ffs(rows) - 1;
+                    rows &= rows - 1;
+                    m = mk[r * DEP_CELLS];
+                    base = r * DEP_TW;
+                }
+                const int k = base + __ffs(m) - 1;
+                m &= m - 1;
+                const double2 pos = s_pos[k], v01 = s_v01[k], v23 = s_v23[k];
+                double wx[3], wy[3];
+                tsc_axis(pos.x, wx[0], wx[1], wx[2]);
+                tsc_axis(pos.y, wy[0], wy[1], wy[2]);
+                const double v[4] = {v01.x, v01.y, v23.x, v23.y};
+#pragma unroll
+                for (int f = 0; f < 4; ++f)
+#pragma unroll
+                    for (int di = 0; di < 3; ++di) {
+                        const double vx = v[f] * wx[di];
+#pragma unroll
+                        for (int dj = 0; dj < 3; ++dj) acc[f][di * 3 + dj] = fma(vx, wy[dj], acc[f][di * 3 + dj]);
+                    }
+            }
+            // (c + 0.5) / mj lies at least 0.5 / mj from an integer, more than the float rounding
+            const int ci = __float2int_rz(((float)c + 0.5f) * inv_mj), cj = c - ci * mj;
+            double* w = s_win + ci * wj + cj;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) {
+                if (any) {
+                    double* we = w + (e / 3) * wj + e % 3;
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) we[f * DEP_WIN] += acc[f][e];
+                }
+                __syncthreads();
+            }
+        }
+
+        // ---- phase 3: split each touched window cell once, add to global ----
+        const float inv_wj = 1.0f / (float)wj;
+        for (int w = t; w < nwin; w += T) {
+            const int ci = __float2int_rz(((float)w + 0.5f) * inv_wj), cj = w - ci * wj;
+            unsigned long long* g = a.acc + (size_t)(oi - 1 + ci) * N + (oj - 1 + cj);
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+                const double v = s_win[f * DEP_WIN + w];
+                if (v != 0.0) fx_add(g + 2 * f * NN, g + (2 * f + 1) * NN, 0, v);
+            }
+        }
+        if (strip + 1 < strips) __syncthreads();   // the window is read; the next one clears it
+    }
 }
 
 // One tile per CTA: blockIdx.x / .y = tile column / row.
 template <int TI>
-__global__ void __launch_bounds__(TI * 32, 1024 / (TI * 32)) deposit_kernel(DepositArgs a) {
+__global__ void __launch_bounds__(dep_threads(TI), 512 / dep_threads(TI)) deposit_kernel(DepositArgs a) {
     deposit_tile<TI>(a, blockIdx.x, blockIdx.y);
 }
 
@@ -662,7 +712,7 @@ __global__ void __launch_bounds__(TI * 32, 1024 / (TI * 32)) deposit_kernel(Depo
 // b - cta_start[s] of simulation s (cta_start: prefix sums of the tile
 // counts, n + 1 entries), whose arguments are args[s].
 template <int TI>
-__global__ void __launch_bounds__(TI * 32, 1024 / (TI * 32))
+__global__ void __launch_bounds__(dep_threads(TI), 512 / dep_threads(TI))
     deposit_multi_kernel(const DepositArgs* __restrict__ args, const int* __restrict__ cta_start, int n) {
     __shared__ DepositArgs sa;
     __shared__ int s_sim;
@@ -683,7 +733,7 @@ __global__ void __launch_bounds__(TI * 32, 1024 / (TI * 32))
     }
     __syncthreads();
     const int t = (int)blockIdx.x - cta_start[s_sim];
-    const int ntx = (sa.Nf + sa.fine_off + 31) / 32;
+    const int ntx = (sa.Nf + sa.fine_off + DEP_TW - 1) / DEP_TW;
     deposit_tile<TI>(sa, t % ntx, t / ntx);
 }
 
@@ -769,11 +819,12 @@ int launch_move_smart(const MoveArgs& a, cudaStream_t s) {
 }
 
 int particles_prepare() {
-    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep2_smem(4)));
-    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep2_smem(8)));
-    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep2_smem(16)));
+    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep_smem<4>()));
+    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep_smem<8>()));
+    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep_smem<12>()));
+    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep_smem<16>()));
     LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_multi_kernel<DEP_MULTI_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)dep2_smem(DEP_MULTI_ROWS)));
+                                       (int)dep_smem<DEP_MULTI_ROWS>()));
     return LC3D_OK;
 }
 
@@ -781,9 +832,9 @@ int particles_prepare() {
 // (lcode.py:468-487) puts two particles per cell and axis, and the pairs of
 // fine indices (odd, even) share a cell, so tiles start one particle early.
 int deposit_fine_offset(int fineness) {
-#ifdef LC3D_DEP2_FORCE_OFF
+#ifdef LC3D_DEP_FORCE_OFF
     (void)fineness;
-    return LC3D_DEP2_FORCE_OFF;
+    return LC3D_DEP_FORCE_OFF;
 #else
     return fineness % 2 == 0 ? 1 : 0;
 #endif
@@ -791,36 +842,27 @@ int deposit_fine_offset(int fineness) {
 
 int launch_deposit_main(const DepositArgs& a, cudaStream_t s) {
     if (a.Nf <= 0) return LC3D_OK;
-    const int ti = a.tile_rows ? a.tile_rows : LC3D_DEP2_ROWS;
-    const dim3 grid2((a.Nf + a.fine_off + 31) / 32, (a.Nf + a.fine_off + ti - 1) / ti);
+    const int ti = a.tile_rows ? a.tile_rows : LC3D_DEP_ROWS;
+    const dim3 grid2((a.Nf + a.fine_off + DEP_TW - 1) / DEP_TW, (a.Nf + a.fine_off + ti - 1) / ti);
     switch (ti) {
-        case 4: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<4>, grid2, dim3(4 * 32), dep2_smem(4), s, a)); break;
-        case 8: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<8>, grid2, dim3(8 * 32), dep2_smem(8), s, a)); break;
-        case 16: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<16>, grid2, dim3(16 * 32), dep2_smem(16), s, a)); break;
+        case 4: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<4>, grid2, dim3(dep_threads(4)), dep_smem<4>(), s, a)); break;
+        case 8: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<8>, grid2, dim3(dep_threads(8)), dep_smem<8>(), s, a)); break;
+        case 12: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<12>, grid2, dim3(dep_threads(12)), dep_smem<12>(), s, a)); break;
+        case 16: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<16>, grid2, dim3(dep_threads(16)), dep_smem<16>(), s, a)); break;
         default: return LC3D_ERR_PARAM;
     }
     LC3D_CUDA_TRY(cudaGetLastError());
     return LC3D_OK;
 }
 
-#if LC3D_DEP2_CLOCKS
-// Instrumented builds only: phase clocks of the last deposit_kernel launch,
-// [16384][DEP2_NCLK] cycles since each CTA's start.
-extern "C" int lc3d_debug_dep_clocks(long long* host) {
-    LC3D_CUDA_TRY(cudaDeviceSynchronize());
-    LC3D_CUDA_TRY(cudaMemcpyFromSymbol(host, g_dep2_clocks, sizeof(g_dep2_clocks)));
-    return LC3D_OK;
-}
-#endif
-
 // Tiles of one simulation's deposition at the multi-simulation tile height.
 int deposit_multi_tiles(const DepositArgs& a) {
-    return ((a.Nf + a.fine_off + 31) / 32) * ((a.Nf + a.fine_off + DEP_MULTI_ROWS - 1) / DEP_MULTI_ROWS);
+    return ((a.Nf + a.fine_off + DEP_TW - 1) / DEP_TW) * ((a.Nf + a.fine_off + DEP_MULTI_ROWS - 1) / DEP_MULTI_ROWS);
 }
 
 int launch_deposit_multi(const DepositArgs* args_dev, const int* cta_start_dev, int n, int ctas, cudaStream_t s) {
     if (n <= 0 || ctas <= 0) return LC3D_OK;
-    deposit_multi_kernel<DEP_MULTI_ROWS><<<ctas, DEP_MULTI_ROWS * 32, dep2_smem(DEP_MULTI_ROWS), s>>>(
+    deposit_multi_kernel<DEP_MULTI_ROWS><<<ctas, dep_threads(DEP_MULTI_ROWS), dep_smem<DEP_MULTI_ROWS>(), s>>>(
         args_dev, cta_start_dev, n);
     LC3D_CUDA_TRY(cudaGetLastError());
     return LC3D_OK;

@@ -220,29 +220,31 @@ constexpr size_t conv_smem_bytes(int cout = 128) {
 //     dW[tap][co][ci] = sum_p g[p][co] x[p + off(tap)][ci]
 // is a GEMM D = A B^T over K = pixels with A[co][p] = g[p][co] and
 // B[ci][p] = x[p + off][ci]. Both operands arrive from the NHWC arrays as
-// TMA boxes of 32 channels x 32 pixels (64-byte rows of channels, 64-byte
+// TMA boxes of 32 channels x 64 pixels (64-byte rows of channels, 64-byte
 // swizzle): channel-contiguous, i.e. MN-major, so the instruction descriptor
 // sets both major bits and the shared-memory descriptors use the canonical
 // MN-major 64-byte-swizzle layout ((4, m), (8, k)) : ((1, LBO), (4, SBO)) in
 // 16-byte units: a 32-channel group is one 64-byte row of a box, the next
-// group (the next box) LBO = 2 KiB further, 8-pixel row groups SBO = 512 bytes
-// apart. M = 128 output channels (rows past Cout are TMA zero fill), N = Cin.
+// group (the next box) LBO = 4 KiB further, 8-pixel row groups SBO = 512 bytes
+// apart. M = 128 output channels, N = Cin.
 // A CTA sums one chunk of pixels for one tap in TMEM (f32) and adds its
 // partial to dW with float32 atomics. The bias gradient stays a plain
 // reduction. Pixels past the level and shifted rows outside it are zero
 // fill; the pad column of g is zero.
 // ---------------------------------------------------------------------------
-constexpr int WG_PIX = 32;                                  // K block: pixels per stage
-constexpr int WG_BOX = 32 * WG_PIX * 2;                     // one 32-channel x 32-pixel box: 2 KiB
+constexpr int WG_PIX = 64;                                  // pixels per stage
+constexpr int WG_ALIGN = 32;                                // chunks are multiples of this
+constexpr int WG_BOX = 32 * WG_PIX * 2;                     // one 32-channel x 64-pixel box: 4 KiB
 constexpr int WG_A_BYTES = 4 * WG_BOX;                      // 128 channels of g
 constexpr int WG_B_MAX = 4 * WG_BOX;                        // up to 128 channels of x
 constexpr int WG_STAGES = 4;
 
 struct WgradArgs {
-    CUtensorMap tg;                // g: [NP][CGp] bf16, box (32 channels, 32 pixels)
-    CUtensorMap tx;                // x: [NP][Cin] bf16, box (32, 32)
+    CUtensorMap tg;                // g: [NP][CGp] bf16, box (32 channels, 64 pixels)
+    CUtensorMap tx;                // x: [NP][Cin] bf16, box (32, 64)
     float* dw;                     // [9][Cout][Cin] float32, accumulated into
-    int Cout, Cin, Wp, NP, chunk;  // chunk: pixels per CTA (a multiple of 32)
+    int Cout, CGp, Cin, Wp, NP;    // CGp: channels of g, Cout or the 32 it is padded to
+    int chunk;                     // pixels per CTA (a multiple of WG_ALIGN)
     uint32_t idesc;
     long long wait_limit;
     unsigned* err;
@@ -278,10 +280,10 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_wgrad_tc_kernel(const __
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tap = blockIdx.y, off = (tap / 3 - 1) * a.Wp + (tap % 3 - 1);
     const int pa = blockIdx.x * a.chunk;
-    const int nkb = (min(a.NP, pa + a.chunk) - pa + WG_PIX - 1) / WG_PIX;
+    const int pixels = min(a.NP, pa + a.chunk) - pa, nkb = (pixels + WG_PIX - 1) / WG_PIX;
     const int nbx = a.Cin / 32;                              // boxes of x per stage
     const uint32_t tcols = (uint32_t)a.Cin;                  // 32, 64 or 128 columns
-    const uint32_t bytes = WG_A_BYTES + (uint32_t)nbx * WG_BOX;
+    const uint32_t bytes = (uint32_t)(a.CGp / 32 + nbx) * WG_BOX;
 
     if (threadIdx.x == 0) {
         s_fail = 0;
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_wgrad_tc_kernel(const __
                 }
                 const int p = pa + kb * WG_PIX;
                 mbar_expect_tx(&full[st], bytes);
-                for (int c = 0; c < 4; ++c)   // channels 32c .. 32c + 31 of g (zero past Cout)
+                for (int c = 0; c < a.CGp / 32; ++c)   // channels 32c .. 32c + 31 of g
                     tma_load_2d(sA + st * WG_A_BYTES + c * WG_BOX, &a.tg, &full[st], 32 * c, p);
                 for (int c = 0; c < nbx; ++c)
                     tma_load_2d(sB + st * WG_B_MAX + c * WG_BOX, &a.tx, &full[st], 32 * c, p + off);
@@ -325,8 +327,9 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_wgrad_tc_kernel(const __
                 fence_after();
                 const uint32_t a_base = smem_u32(sA + st * WG_A_BYTES);
                 const uint32_t b_base = smem_u32(sB + st * WG_B_MAX);
-#pragma unroll
-                for (int kk = 0; kk < WG_PIX / 16; ++kk)   // 16 pixels (two 8-row groups) per MMA
+                // 16 pixels (two 8-row groups) per MMA, up to the chunk's end
+                const int nkk = min(WG_PIX, (pixels - kb * WG_PIX + 15) / 16 * 16) / 16;
+                for (int kk = 0; kk < nkk; ++kk)
                     umma_bf16(tmem, umma_desc_mn_sw64(a_base + kk * 1024, WG_BOX),
                               umma_desc_mn_sw64(b_base + kk * 1024, WG_BOX), a.idesc, (kb | kk) ? 1u : 0u);
                 umma_commit(&empty[st]);
@@ -586,34 +589,6 @@ __global__ void target_kernel(const __grid_constant__ OutArgs a) {
     for (int q = 0; q < 4; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
 }
 
-// Mean squared error over the 5 used channels of the H x W pixels; g = dL/dy.
-__global__ void loss_kernel(const float* __restrict__ y, const float* __restrict__ t, float* __restrict__ g,
-                            Level L, float* loss) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const float inv = 1.0f / (5.0f * (float)L.H * (float)L.W);
-    float s = 0.0f;
-    if (p < L.NP) {
-        const int x = p % L.Wp;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-            float d = 0.0f;
-            if (c < 5 && x < L.W) d = y[(size_t)p * 16 + c] - t[(size_t)p * 16 + c];
-            s += d * d;
-            g[(size_t)p * 16 + c] = 2.0f * d * inv;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __shared__ float ws[32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float b = 0.0f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) b += ws[w];
-        atomicAdd(loss, b * inv);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Backward data pass on the tensor cores. dL/dx of a 3x3 convolution is the
 // 3x3 convolution of the output gradient g with the flipped, transposed
@@ -623,17 +598,6 @@ __global__ void loss_kernel(const float* __restrict__ y, const float* __restrict
 // column), the accumulation is f32 in TMEM, and the epilogue applies the
 // ReLU adjoint of the layer's input.
 // ---------------------------------------------------------------------------
-
-// out[p][c] = bf16(g[p][c]) for c < CG and real pixels; 0 for c >= CG and
-// in the pad column.
-__global__ void grad_to_bf16_kernel(const float* __restrict__ g, int CG, __nv_bfloat16* __restrict__ out, int CGp,
-                                    Level L) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)L.NP * CGp) return;
-    const int p = (int)(t / CGp), c = (int)(t - (long long)p * CGp);
-    const bool pad = (p % L.Wp) >= L.W;
-    out[t] = __float2bfloat16_rn(!pad && c < CG ? g[(size_t)p * CG + c] : 0.0f);
-}
 
 // wt[tap][ci][co] = w[8 - tap][co][ci] (co < CG), 0 for CG <= co < CGp.
 __global__ void flip_weights_kernel(const __nv_bfloat16* __restrict__ w, int CG, int CIN, int CGp,
@@ -649,49 +613,166 @@ __global__ void flip_weights_kernel(const __nv_bfloat16* __restrict__ w, int CG,
 // adjoints and Adam
 // ---------------------------------------------------------------------------
 
-// db[co] += sum_p g[p][co] over one chunk of pixels.
-__global__ void bias_grad_kernel(const float* __restrict__ g, int CG, float* __restrict__ db, int NP, int chunk) {
-    const int pa = blockIdx.x * chunk, pb = min(NP, pa + chunk);
-    for (int co = threadIdx.x; co < CG; co += blockDim.x) {
-        float s = 0.0f;
-        for (int p = pa; p < pb; ++p) s += g[(size_t)p * CG + co];
-        atomicAdd(db + co, s);
+// The kernels that produce a layer's output gradient write it in bf16, the
+// operand of both tensor-core passes (0 in the pad column and past CG
+// channels), and add its sums over the pixels to the bias gradient db on the
+// way: a thread has 8 channels of every few hundredth pixel, a CTA adds its
+// sums by float32 atomics. (A separate bias kernel, 128 CTAs walking the
+// float32 gradient pixel by pixel, took 970 of the 2200 us of a training
+// sample at 641^2, a separate conversion 160.)
+constexpr int GRAD_THREADS = 256;
+
+// s[8] of every thread, thread t holding channel group t % G, summed over the
+// CTA into db[0 .. 8 G). G = 4, 8 or 16.
+__device__ __forceinline__ void add_bias_sums(float (&s)[8], int G, float* db) {
+    __shared__ float ws[GRAD_THREADS / 32][128];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int o = 16; o >= G; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+    if (lane < G)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ws[warp][lane * 8 + j] = s[j];
+    __syncthreads();
+    if ((int)threadIdx.x < 8 * G) {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < GRAD_THREADS / 32; ++w) v += ws[w][threadIdx.x];
+        atomicAdd(db + threadIdx.x, v);
     }
 }
 
-// g_u[Y][X][c] = sum of g_d over the valid fine children (adjoint of the
-// nearest-neighbour upsampling).
-__global__ void downsum_kernel(const float* __restrict__ gd, Level lf, float* __restrict__ gu, Level lc, int C) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)lc.NP * C) return;
-    const int p = (int)(t / C), c = (int)(t - (long long)p * C);
-    const int Y = p / lc.Wp, X = p - Y * lc.Wp;
-    float s = 0.0f;
-    if (X < lc.W)
-        for (int dy = 0; dy < 2; ++dy)
-            for (int dx = 0; dx < 2; ++dx) {
-                const int y = 2 * Y + dy, x = 2 * X + dx;
-                if (y < lf.H && x < lf.W) s += gd[((size_t)y * lf.Wp + x) * C + c];
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// Mean squared error over the 5 used channels of the H x W pixels and its
+// gradient: g[p][0 .. 32) = dL/dy, a thread per pixel.
+__global__ void __launch_bounds__(GRAD_THREADS) loss_kernel(const float* __restrict__ y, const float* __restrict__ t,
+                                                            __nv_bfloat16* __restrict__ g, Level L, float* loss,
+                                                            float* __restrict__ db) {
+    const float inv = 1.0f / (5.0f * (float)L.H * (float)L.W);
+    float sq = 0.0f, s[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    for (int p = blockIdx.x * GRAD_THREADS + threadIdx.x; p < L.NP; p += gridDim.x * GRAD_THREADS) {
+        float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (p % L.Wp < L.W) {
+            float a[8], b[8];
+            load8(y + (size_t)p * 16, a);
+            load8(t + (size_t)p * 16, b);
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                const float d = a[c] - b[c];
+                sq += d * d;
+                v[c] = 2.0f * d * inv;
+                s[c] += v[c];
             }
-    gu[t] = s;
+        }
+        uint4* o = reinterpret_cast<uint4*>(g + (size_t)p * 32);
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        o[0] = pack_bf8(v);
+        o[1] = zero;
+        o[2] = zero;
+        o[3] = zero;
+    }
+    __shared__ float ws[GRAD_THREADS / 32][6];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        sq += __shfl_xor_sync(0xffffffffu, sq, o);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int c = 0; c < 5; ++c) ws[warp][c] = s[c];
+        ws[warp][5] = sq;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < GRAD_THREADS / 32; ++w) v += ws[w][threadIdx.x];
+        if (threadIdx.x < 5) atomicAdd(db + threadIdx.x, v);
+        else atomicAdd(loss, v * inv);
+    }
 }
 
-// g_e = (g_e + g_p[parent] / children(parent)) * (e > 0) (adjoint of the
-// average pooling, plus the skip gradient already in g_e, through the ReLU).
-__global__ void pool_bwd_mask_kernel(float* __restrict__ ge, const __nv_bfloat16* __restrict__ e, Level lf,
-                                     const float* __restrict__ gp, Level lc, int C) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)lf.NP * C) return;
-    const int p = (int)(t / C), c = (int)(t - (long long)p * C);
-    const int y = p / lf.Wp, x = p - y * lf.Wp;
-    float v = 0.0f;
-    if (x < lf.W) {
-        const int Y = y >> 1, X = x >> 1;
-        const int cnt = (min(2 * Y + 2, lf.H) - 2 * Y) * (min(2 * X + 2, lf.W) - 2 * X);
-        v = ge[t] + gp[((size_t)Y * lc.Wp + X) * C + c] / (float)cnt;
-        if (!(__bfloat162float(e[t]) > 0.0f)) v = 0.0f;
+// out = bf16(g), C channels.
+__global__ void __launch_bounds__(GRAD_THREADS) grad_bf16_kernel(const float* __restrict__ g, __nv_bfloat16* __restrict__ out,
+                                                                 Level L, int C, float* __restrict__ db) {
+    const int G = C / 8, c = threadIdx.x % G * 8, per = GRAD_THREADS / G;
+    float s[8] = {};
+    for (int p = blockIdx.x * per + threadIdx.x / G; p < L.NP; p += gridDim.x * per) {
+        float v[8] = {};
+        if (p % L.Wp < L.W) {
+            load8(g + (size_t)p * C + c, v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[j] += v[j];
+        }
+        *reinterpret_cast<uint4*>(out + (size_t)p * C + c) = pack_bf8(v);
     }
-    ge[t] = v;
+    add_bias_sums(s, G, db);
+}
+
+// out[Y][X][c] = sum of g_d over the valid fine children (adjoint of the
+// nearest-neighbour upsampling).
+__global__ void __launch_bounds__(GRAD_THREADS) downsum_kernel(const float* __restrict__ gd, Level lf,
+                                                               __nv_bfloat16* __restrict__ out, Level lc, int C,
+                                                               float* __restrict__ db) {
+    const int G = C / 8, c = threadIdx.x % G * 8, per = GRAD_THREADS / G;
+    float s[8] = {};
+    for (int p = blockIdx.x * per + threadIdx.x / G; p < lc.NP; p += gridDim.x * per) {
+        const int Y = p / lc.Wp, X = p - Y * lc.Wp;
+        float v[8] = {};
+        if (X < lc.W) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int y = 2 * Y + k / 2, x = 2 * X + k % 2;
+                if (y < lf.H && x < lf.W) {
+                    float w[8];
+                    load8(gd + ((size_t)y * lf.Wp + x) * C + c, w);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[j] += w[j];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[j] += v[j];
+        }
+        *reinterpret_cast<uint4*>(out + (size_t)p * C + c) = pack_bf8(v);
+    }
+    add_bias_sums(s, G, db);
+}
+
+// out = (g_e + g_p[parent] / children(parent)) * (e > 0) (adjoint of the
+// average pooling, plus the skip gradient in g_e, through the ReLU).
+__global__ void __launch_bounds__(GRAD_THREADS) pool_bwd_mask_kernel(const float* __restrict__ ge,
+                                                                     const __nv_bfloat16* __restrict__ e, Level lf,
+                                                                     const float* __restrict__ gp, Level lc, int C,
+                                                                     __nv_bfloat16* __restrict__ out,
+                                                                     float* __restrict__ db) {
+    const int G = C / 8, c = threadIdx.x % G * 8, per = GRAD_THREADS / G;
+    float s[8] = {};
+    for (int p = blockIdx.x * per + threadIdx.x / G; p < lf.NP; p += gridDim.x * per) {
+        const int y = p / lf.Wp, x = p - y * lf.Wp;
+        float v[8] = {};
+        if (x < lf.W) {
+            const int Y = y >> 1, X = x >> 1;
+            const int cnt = (min(2 * Y + 2, lf.H) - 2 * Y) * (min(2 * X + 2, lf.W) - 2 * X);
+            float w[8], act[8];
+            load8(ge + (size_t)p * C + c, v);
+            load8(gp + ((size_t)Y * lc.Wp + X) * C + c, w);
+            unpack_bf8(__ldg(reinterpret_cast<const uint4*>(e + (size_t)p * C + c)), act);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[j] = act[j] > 0.0f ? v[j] + w[j] / (float)cnt : 0.0f;
+                s[j] += v[j];
+            }
+        }
+        *reinterpret_cast<uint4*>(out + (size_t)p * C + c) = pack_bf8(v);
+    }
+    add_bias_sums(s, G, db);
 }
 
 // Adam on the float32 master parameters; refreshes the bf16 copy.
@@ -771,8 +852,7 @@ struct lc3d_predictor {
                   *u3 = nullptr, *d2 = nullptr, *u2 = nullptr, *d1 = nullptr;
     float *y = nullptr, *target = nullptr;
     // gradients (float32 NHWC)
-    float *g_out = nullptr, *g_d1 = nullptr, *g_u2 = nullptr, *g_d2 = nullptr, *g_u3 = nullptr, *g_e3 = nullptr,
-          *g_p2 = nullptr, *g_p1 = nullptr;
+    float *g_d1 = nullptr, *g_d2 = nullptr, *g_e3 = nullptr, *g_p2 = nullptr, *g_p1 = nullptr;
     // tensor-core backward data pass: the bf16 output gradient of the layer
     // in hand, the flipped transposed bf16 weights of every layer, zeros for
     // the bias, and the convolution arguments of each layer's pass
@@ -782,7 +862,7 @@ struct lc3d_predictor {
     float* zero_bias = nullptr;
     ConvArgs bconv[NLAYERS];
     WgradArgs wg[NLAYERS];         // tensor-core weight gradient of each layer
-    int wg_chunks[NLAYERS];
+    dim3 wg_grid[NLAYERS];
     unsigned* err = nullptr;
     double* scale = nullptr;       // [23] per-sample channel scales (device)
     double* partial = nullptr;     // [STAT_BLOCKS][18]
@@ -849,17 +929,6 @@ int setup_bconv(lc3d_predictor* P, int l) {
     return LC3D_OK;
 }
 
-// Layer l's output gradient g (float32) as bf16 in P->g_bf: the operand of
-// both tensor-core passes of the layer.
-int grad_bf16(lc3d_predictor* P, int l, const float* g, cudaStream_t s) {
-    const LayerDef& d = LAYERS[l];
-    const Level& L = P->lv[d.level];
-    const int CGp = grad_channels(l);
-    grad_to_bf16_kernel<<<blocks_for((long long)L.NP * CGp, 256), 256, 0, s>>>(g, d.cout, P->g_bf, CGp, L);
-    LC3D_CUDA_TRY(cudaGetLastError());
-    return LC3D_OK;
-}
-
 int setup_wgrad(lc3d_predictor* P, int l, const __nv_bfloat16* x) {
     const LayerDef& d = LAYERS[l];
     const Level& L = P->lv[d.level];
@@ -869,33 +938,29 @@ int setup_wgrad(lc3d_predictor* P, int l, const __nv_bfloat16* x) {
     LC3D_TRY(make_map_2d(&a.tx, x, L.NP, d.cin, WG_PIX));
     a.dw = P->grad + P->w_off[l];
     a.Cout = d.cout;
+    a.CGp = grad_channels(l);
     a.Cin = d.cin;
     a.Wp = L.Wp;
     a.NP = L.NP;
-    // 16 pixel chunks per tap (9 x 16 CTAs), each a multiple of the K block
-    const int chunks = (int)std::min<long long>(16, (L.NP + WG_PIX - 1) / WG_PIX);
-    a.chunk = (int)(((L.NP + chunks - 1) / chunks + WG_PIX - 1) / WG_PIX * WG_PIX);
-    P->wg_chunks[l] = (L.NP + a.chunk - 1) / a.chunk;
+    // 16 pixel chunks per tap: 9 x 16 CTAs
+    const int chunks = (int)std::min<long long>(16, (L.NP + WG_ALIGN - 1) / WG_ALIGN);
+    a.chunk = (int)(((L.NP + chunks - 1) / chunks + WG_ALIGN - 1) / WG_ALIGN * WG_ALIGN);
+    P->wg_grid[l] = dim3((L.NP + a.chunk - 1) / a.chunk, 9);
     a.idesc = idesc_bf16_mn(128, d.cin);
     a.wait_limit = WAIT_LIMIT;
     a.err = P->err;
     return LC3D_OK;
 }
 
-// dW of layer l from P->g_bf (grad_bf16 first) and the bias gradient from g.
-int bwd_weights_tc(lc3d_predictor* P, int l, const float* g, cudaStream_t s) {
+// dW of layer l from its output gradient in P->g_bf.
+int bwd_weights_tc(lc3d_predictor* P, int l, cudaStream_t s) {
     const WgradArgs& a = P->wg[l];
-    conv_wgrad_tc_kernel<<<dim3(P->wg_chunks[l], 9), CONV_THREADS, wgrad_smem_bytes(), s>>>(a);
-    LC3D_CUDA_TRY(cudaGetLastError());
-    const Level& L = P->lv[LAYERS[l].level];
-    const int nchunks = (int)std::min<long long>(128, (L.NP + 1023) / 1024);
-    const int chunk = (L.NP + nchunks - 1) / nchunks;
-    bias_grad_kernel<<<(L.NP + chunk - 1) / chunk, 128, 0, s>>>(g, LAYERS[l].cout, P->grad + P->b_off[l], L.NP, chunk);
+    conv_wgrad_tc_kernel<<<P->wg_grid[l], CONV_THREADS, wgrad_smem_bytes(), s>>>(a);
     LC3D_CUDA_TRY(cudaGetLastError());
     return LC3D_OK;
 }
 
-// dx = dL/d(input of layer l) from P->g_bf (grad_bf16 first), zeroed where mask <= 0.
+// dx = dL/d(input of layer l) from P->g_bf, zeroed where mask <= 0.
 int bwd_data_tc(lc3d_predictor* P, int l, const __nv_bfloat16* mask, float* dx, cudaStream_t s) {
     ConvArgs a = P->bconv[l];
     a.out = dx;
@@ -931,33 +996,35 @@ int backward(lc3d_predictor* P, float* loss, cudaStream_t s) {
                                                                 grad_channels(l), P->wt + P->wt_off[l]);
     }
     LC3D_CUDA_TRY(cudaGetLastError());
-    // each layer: its output gradient in bf16 once, then the weight and data passes on it
-#define LC3D_BWD_W(l, CG, CIN, g, x) LC3D_TRY(grad_bf16(P, l, g, s)); LC3D_TRY(bwd_weights_tc(P, l, g, s))
-#define LC3D_BWD_DATA(l, CIN, g, CG, mask, dx, lev) LC3D_TRY(bwd_data_tc(P, l, mask, dx, s))
-    loss_kernel<<<blocks_for(l0.NP, 256), 256, 0, s>>>(P->y, P->target, P->g_out, l0, loss);
+    // each layer: its output gradient in bf16 (P->g_bf) with the bias
+    // gradient, then the weight and data passes on it
+    auto db = [&](int l) { return P->grad + P->b_off[l]; };
+    auto grid = [&](const Level& L, int C) {   // CTAs of a gradient kernel: a few pixels per thread, six CTAs per SM at most
+        return std::min(blocks_for((long long)L.NP * (C / 8), GRAD_THREADS * 4), 148u * 6);
+    };
     // conv6: d1 -> y
-    LC3D_BWD_W(5, 16, 32, P->g_out, P->d1);
-    LC3D_BWD_DATA(5, 32, P->g_out, 16, P->d1, P->g_d1, l0);
-    downsum_kernel<<<blocks_for((long long)l1.NP * 32, 256), 256, 0, s>>>(P->g_d1, l0, P->g_u2, l1, 32);
+    loss_kernel<<<grid(l0, 8), GRAD_THREADS, 0, s>>>(P->y, P->target, P->g_bf, l0, loss, db(5));
+    LC3D_TRY(bwd_weights_tc(P, 5, s));
+    LC3D_TRY(bwd_data_tc(P, 5, P->d1, P->g_d1, s));
     // conv5: d2 -> u2
-    LC3D_BWD_W(4, 32, 64, P->g_u2, P->d2);
-    LC3D_BWD_DATA(4, 64, P->g_u2, 32, P->d2, P->g_d2, l1);
-    downsum_kernel<<<blocks_for((long long)l2.NP * 64, 256), 256, 0, s>>>(P->g_d2, l1, P->g_u3, l2, 64);
+    downsum_kernel<<<grid(l1, 32), GRAD_THREADS, 0, s>>>(P->g_d1, l0, P->g_bf, l1, 32, db(4));
+    LC3D_TRY(bwd_weights_tc(P, 4, s));
+    LC3D_TRY(bwd_data_tc(P, 4, P->d2, P->g_d2, s));
     // conv4: e3 -> u3
-    LC3D_BWD_W(3, 64, 128, P->g_u3, P->e3);
-    LC3D_BWD_DATA(3, 128, P->g_u3, 64, P->e3, P->g_e3, l2);
+    downsum_kernel<<<grid(l2, 64), GRAD_THREADS, 0, s>>>(P->g_d2, l1, P->g_bf, l2, 64, db(3));
+    LC3D_TRY(bwd_weights_tc(P, 3, s));
+    LC3D_TRY(bwd_data_tc(P, 3, P->e3, P->g_e3, s));
     // conv3: p2 -> e3
-    LC3D_BWD_W(2, 128, 64, P->g_e3, P->p2);
-    LC3D_BWD_DATA(2, 64, P->g_e3, 128, nullptr, P->g_p2, l2);
-    pool_bwd_mask_kernel<<<blocks_for((long long)l1.NP * 64, 256), 256, 0, s>>>(P->g_d2, P->e2, l1, P->g_p2, l2, 64);
-    // conv2: p1 -> e2 (g_d2 now holds dL/d pre-activation of e2)
-    LC3D_BWD_W(1, 64, 32, P->g_d2, P->p1);
-    LC3D_BWD_DATA(1, 32, P->g_d2, 64, nullptr, P->g_p1, l1);
-    pool_bwd_mask_kernel<<<blocks_for((long long)l0.NP * 32, 256), 256, 0, s>>>(P->g_d1, P->e1, l0, P->g_p1, l1, 32);
+    grad_bf16_kernel<<<grid(l2, 128), GRAD_THREADS, 0, s>>>(P->g_e3, P->g_bf, l2, 128, db(2));
+    LC3D_TRY(bwd_weights_tc(P, 2, s));
+    LC3D_TRY(bwd_data_tc(P, 2, nullptr, P->g_p2, s));
+    // conv2: p1 -> e2
+    pool_bwd_mask_kernel<<<grid(l1, 64), GRAD_THREADS, 0, s>>>(P->g_d2, P->e2, l1, P->g_p2, l2, 64, P->g_bf, db(1));
+    LC3D_TRY(bwd_weights_tc(P, 1, s));
+    LC3D_TRY(bwd_data_tc(P, 1, nullptr, P->g_p1, s));
     // conv1: x0 -> e1
-    LC3D_BWD_W(0, 32, 32, P->g_d1, P->x0);
-#undef LC3D_BWD_W
-#undef LC3D_BWD_DATA
+    pool_bwd_mask_kernel<<<grid(l0, 32), GRAD_THREADS, 0, s>>>(P->g_d1, P->e1, l0, P->g_p1, l1, 32, P->g_bf, db(0));
+    LC3D_TRY(bwd_weights_tc(P, 0, s));
     LC3D_CUDA_TRY(cudaGetLastError());
     return LC3D_OK;
 }
@@ -1001,16 +1068,15 @@ int lc3d_predictor_create(int grid_steps, int device, lc3d_predictor** out) {
     PA(P->x0, n0 * 32); PA(P->e1, n0 * 32); PA(P->p1, n1 * 32); PA(P->e2, n1 * 64); PA(P->p2, n2 * 64);
     PA(P->e3, n2 * 128); PA(P->u3, n2 * 64); PA(P->d2, n1 * 64); PA(P->u2, n1 * 32); PA(P->d1, n0 * 32);
     PA(P->y, n0 * 16); PA(P->target, n0 * 16);
-    PA(P->g_out, n0 * 16); PA(P->g_d1, n0 * 32); PA(P->g_u2, n1 * 32); PA(P->g_d2, n1 * 64);
-    PA(P->g_u3, n2 * 64); PA(P->g_e3, n2 * 128); PA(P->g_p2, n2 * 64); PA(P->g_p1, n1 * 32);
+    PA(P->g_d1, n0 * 32); PA(P->g_d2, n1 * 64); PA(P->g_e3, n2 * 128); PA(P->g_p2, n2 * 64); PA(P->g_p1, n1 * 32);
     PA(P->err, 1); PA(P->scale, 23); PA(P->partial, (size_t)STAT_BLOCKS * 18);
     {   // tensor-core backward data pass (layers 2..6; the input gradient of layer 1 is not needed)
         size_t gmax = 0;
         long long wtot = 0;
         for (int l = 0; l < NLAYERS; ++l) {
             P->wt_off[l] = wtot;
-            if (l == 0) continue;
             gmax = std::max(gmax, (size_t)P->lv[LAYERS[l].level].NP * grad_channels(l));
+            if (l == 0) continue;
             wtot += 9LL * LAYERS[l].cin * grad_channels(l);
         }
         PA(P->g_bf, gmax); PA(P->wt, (size_t)wtot); PA(P->zero_bias, 128);

@@ -1,4 +1,7 @@
-// Spectral field solvers in dense-transform (GEMM) form, float64.
+// Spectral field solvers: right-hand sides, eigenvalues, the choice of the
+// transforms' form (float64 FFT: fields_fft64.cu, float64 dense:
+// fields_dense.cu, float32 FFT: fields_fft.cu, split tensor-core GEMMs:
+// fields_mixed.cu) and the step finalize.
 //
 // Reference: lcode.py:124-184 (dst2d, dirichlet_matrix, calculate_Ez),
 // 187-290 (mix2d, mixed_matrix, dx_dy, calculate_Ex_Ey_Bx_By), 293-364
@@ -17,7 +20,7 @@
 //   Ez:     X = rhs_inner         L = S2, R = S2,  Lambda = dirichlet_matrix
 //   Bz:     X = rhs               L = C,  R = C^T, Lambda = neumann_matrix
 //           (dct2d is minus the DCT-I; the two signs cancel)
-// All six fields of a solve run as one batched GEMM per stage (4 stages).
+// All six fields of a solve run in each launch.
 
 #include <cmath>
 #include <cstring>
@@ -111,150 +114,6 @@ __global__ void __launch_bounds__(RHS_THREADS) rhs_kernel(const __grid_constant_
 #pragma unroll
     for (int f = 0; f < 6; ++f)
         if (a.out[f]) a.out[f][k] = o[f];
-}
-
-// ---------------------------------------------------------------------------
-// Batched float64 GEMM, C = A B (optionally C = Lambda o (A B)), row-major,
-// on the float64 tensor cores (mma.sync m8n8k4 .f64: each product and sum is
-// an IEEE float64 fused multiply-add). 128 x 64 tiles per 256-thread CTA,
-// eight warps in a 4 x 2 grid of 32 x 32 warp tiles (4 x 4 MMAs per k4
-// step); k-steps of 16 staged by cp.async into two shared-memory buffers,
-// the next k-step copied while the current one is multiplied.
-// ---------------------------------------------------------------------------
-constexpr int MAX_PROBS = 6;
-
-struct GemmProb {
-    const double *A, *B, *L;
-    double* C;
-    int M, N, K, lda, ldb, ldc, ldl;
-    int tiles_n, tile_start;
-};
-
-struct GemmBatch {
-    GemmProb p[MAX_PROBS];
-    int count, total_tiles;
-};
-
-constexpr int GTM = 128, GTN = 64, GK = 16;
-constexpr int GEMM_THREADS = 256;
-// shared pitches (doubles): the fragment loads of a half-warp (rows g = 0..3
-// or 4..7, columns t = 0..3) fall in distinct banks: 2 (20 g + t) and
-// 2 (68 t + g) mod 32 are distinct over the 16 lanes
-constexpr int AS_LD = GK + 4;    // As[m][k]
-constexpr int BS_LD = GTN + 4;   // Bs[k][n]
-constexpr int AS_SIZE = GTM * AS_LD, BS_SIZE = GK * BS_LD;
-constexpr size_t GEMM_SMEM = 2 * (size_t)(AS_SIZE + BS_SIZE) * sizeof(double);
-
-// 8-byte global -> shared copy; a source size of 0 writes zeros (the tile
-// edges past M, N or K).
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool in) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(in ? 8 : 0) : "memory");
-}
-
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
-}
-
-__global__ void __launch_bounds__(GEMM_THREADS, 2) dgemm_kernel(const __grid_constant__ GemmBatch b) {
-    extern __shared__ __align__(16) double gsm[];   // As[2][GTM][AS_LD], Bs[2][GK][BS_LD]
-    double* As = gsm;
-    double* Bs = gsm + 2 * AS_SIZE;
-    const int bid = blockIdx.x;
-    int pi = 0;
-#pragma unroll 1
-    for (int q = 1; q < b.count; ++q)
-        if (bid >= b.p[q].tile_start) pi = q;
-    const GemmProb& P = b.p[pi];
-    const int t = bid - P.tile_start;
-    const int tm = t / P.tiles_n, tn = t - tm * P.tiles_n;
-    const int row0 = tm * GTM, col0 = tn * GTN;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, tq = lane & 3;            // fragment row group, thread in group
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-
-    auto load = [&](int k0, int buf) {
-        double* as = As + buf * AS_SIZE;
-        double* bs = Bs + buf * BS_SIZE;
-#pragma unroll
-        for (int i = 0; i < GTM * GK / GEMM_THREADS; ++i) {   // 8: rows idx / 16, k idx % 16
-            const int idx = tid + i * GEMM_THREADS, r = idx >> 4, kk = idx & 15;
-            const int row = row0 + r, k = k0 + kk;
-            const bool in = row < P.M && k < P.K;
-            cp_async8(as + r * AS_LD + kk, in ? P.A + (size_t)row * P.lda + k : P.A, in);
-        }
-#pragma unroll
-        for (int i = 0; i < GK * GTN / GEMM_THREADS; ++i) {   // 4: k rows idx / 64, columns idx % 64
-            const int idx = tid + i * GEMM_THREADS, kk = idx >> 6, n = idx & 63;
-            const int k = k0 + kk, col = col0 + n;
-            const bool in = k < P.K && col < P.N;
-            cp_async8(bs + kk * BS_LD + n, in ? P.B + (size_t)k * P.ldb + col : P.B, in);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-
-    double acc[4][4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-    const int nk = (P.K + GK - 1) / GK;
-    load(0, 0);
-    for (int kt = 0; kt < nk; ++kt) {
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();   // k-step kt is in; every warp is done with the other buffer
-        if (kt + 1 < nk) load((kt + 1) * GK, (kt + 1) & 1);
-        const double* as = As + (kt & 1) * AS_SIZE + (wm + g) * AS_LD + tq;
-        const double* bs = Bs + (kt & 1) * BS_SIZE + tq * BS_LD + wn + g;
-#pragma unroll
-        for (int ks = 0; ks < GK; ks += 4) {
-            double af[4], bf[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) af[i] = as[i * 8 * AS_LD + ks];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bf[j] = bs[ks * BS_LD + j * 8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dmma(acc[i][j], af[i], bf[j]);
-        }
-    }
-    // accumulator (i, j, h): row wm + 8 i + g, column wn + 8 j + 2 tq + h
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int row = row0 + wm + 8 * i + g;
-        if (row >= P.M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int col = col0 + wn + 8 * j + 2 * tq + h;
-                if (col >= P.N) continue;
-                double v = acc[i][j][h];
-                if (P.L) v *= P.L[(size_t)row * P.ldl + col];
-                P.C[(size_t)row * P.ldc + col] = v;
-            }
-        }
-    }
-}
-
-int launch_gemm(lc3d_ctx* c, GemmBatch& b, cudaStream_t s) {
-    int tiles = 0;
-    for (int q = 0; q < b.count; ++q) {
-        GemmProb& p = b.p[q];
-        p.tiles_n = (p.N + GTN - 1) / GTN;
-        p.tile_start = tiles;
-        tiles += ((p.M + GTM - 1) / GTM) * p.tiles_n;
-    }
-    b.total_tiles = tiles;
-    if (tiles == 0) return LC3D_OK;
-    ProfScope ps(c, LC3D_STAGE_TRANSFORM, s);
-    dgemm_kernel<<<tiles, GEMM_THREADS, GEMM_SMEM, s>>>(b);
-    LC3D_CUDA_TRY(cudaGetLastError());
-    return LC3D_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -371,18 +230,8 @@ __global__ void __launch_bounds__(RED_THREADS) subtract_mean_kernel(double* a, i
 }
 
 // ---------------------------------------------------------------------------
-// Host: transform and eigenvalue matrices.
+// Host: eigenvalue matrices.
 // ---------------------------------------------------------------------------
-
-// sin(pi r / L) for integer r, with the argument reduced to [0, pi/2].
-double sin_pi_frac(long long r, long long L) {
-    r %= 2 * L;
-    if (r < 0) r += 2 * L;
-    double sign = 1;
-    if (r >= L) { r -= L; sign = -1; }
-    if (2 * r > L) r = L - r;
-    return sign * std::sin(M_PI * (double)r / (double)L);
-}
 
 // lam[k] = 4 / h**2 * sin(k pi / (2 (N - 1)))**2 as lcode.py:152-154 writes it
 double lam(int k, int N, double h) {
@@ -407,22 +256,8 @@ int upload32(float** dst, const std::vector<double>& v) {
 }  // namespace
 
 int fields_init(lc3d_ctx* c) {
-    LC3D_CUDA_TRY(cudaFuncSetAttribute(dgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
     const int N = c->N, M = c->M;
-    const long long L = N - 1;
     const double h = c->p.grid_step_size;
-    std::vector<double> S2((size_t)M * M), C((size_t)N * N), CT((size_t)N * N);
-    for (int k = 0; k < M; ++k)
-        for (int n = 0; n < M; ++n) S2[(size_t)k * M + n] = 2 * sin_pi_frac((long long)(k + 1) * (n + 1), L);
-    for (int k = 0; k < N; ++k)
-        for (int n = 0; n < N; ++n) {
-            // cos(pi r / L) = sin(pi (2 r + L) / (2 L)), r = k n mod 2L
-            const long long r = ((long long)k * n) % (2 * L);
-            const double cv = sin_pi_frac(2 * r + L, 2 * L);
-            const double w = (n == 0 || n == N - 1) ? 1.0 : 2.0;
-            C[(size_t)k * N + n] = w * cv;
-            CT[(size_t)n * N + k] = w * cv;
-        }
     const double norm = 1.0 / ((2.0 * (N - 1)) * (2.0 * (N - 1)));
     const double trick = c->p.field_solver_subtraction_trick != 0 ? 1.0 : 0.0;
     std::vector<double> ld((size_t)M * M), lm((size_t)M * N), lmT((size_t)N * M), ln((size_t)N * N);
@@ -439,9 +274,6 @@ int fields_init(lc3d_ctx* c) {
     for (int i = 0; i < N; ++i)
         for (int j = 0; j < N; ++j)
             ln[(size_t)i * N + j] = (i == 0 && j == 0) ? 0.0 : (1 / (lamk[i] + lamk[j])) * norm;
-    LC3D_TRY(upload(&c->S2, S2));
-    LC3D_TRY(upload(&c->C, C));
-    LC3D_TRY(upload(&c->CT, CT));
     LC3D_TRY(upload(&c->lam_dir, ld));
     LC3D_TRY(upload(&c->lam_mix, lm));
     LC3D_TRY(upload(&c->lam_mixT, lmT));
@@ -471,7 +303,7 @@ int fields_init(lc3d_ctx* c) {
 }
 
 void fields_free(lc3d_ctx* c) {
-    double** ps[] = {&c->S2, &c->C, &c->CT, &c->lam_dir, &c->lam_mix, &c->lam_mixT, &c->lam_neu, &c->red};
+    double** ps[] = {&c->lam_dir, &c->lam_mix, &c->lam_mixT, &c->lam_neu, &c->red};
     for (double** p : ps) {
         if (*p) cudaFree(*p);
         *p = nullptr;
@@ -495,8 +327,8 @@ namespace {
 struct FieldGeom {
     int rows, cols;
     size_t off;            // offset of X / output inside an N x N plane
-    const double *L, *R, *Lam;
-    int ldL, ldR, ldLam;
+    const double* Lam;
+    int ldLam;
     int type0, type1;      // axis-0 / axis-1 transform: 0 DCT-I, 1 DST-I
 };
 
@@ -505,16 +337,16 @@ FieldGeom geom(const lc3d_ctx* c, int f) {
     FieldGeom g{};
     switch (f) {
         case 0: case 4:   // Ex, By: solved transposed
-            g = {N, M, 1, c->C, c->S2, c->lam_mixT, N, M, M, 0, 1};
+            g = {N, M, 1, c->lam_mixT, M, 0, 1};
             break;
         case 1: case 3:   // Ey, Bx
-            g = {M, N, (size_t)N, c->S2, c->CT, c->lam_mix, M, N, N, 1, 0};
+            g = {M, N, (size_t)N, c->lam_mix, N, 1, 0};
             break;
         case 2:           // Ez
-            g = {M, M, (size_t)N + 1, c->S2, c->S2, c->lam_dir, M, M, M, 1, 1};
+            g = {M, M, (size_t)N + 1, c->lam_dir, M, 1, 1};
             break;
         default:          // Bz
-            g = {N, N, 0, c->C, c->CT, c->lam_neu, N, N, N, 0, 0};
+            g = {N, N, 0, c->lam_neu, N, 0, 0};
             break;
     }
     return g;
@@ -715,44 +547,14 @@ int solve_fields(lc3d_ctx* c, int which, const SolveInputs& in, const SolveOutpu
             }
         }
     } else {
-        // the four GEMM stages
-        for (int stage = 0; stage < 4; ++stage) {
-            GemmBatch b{};
-            memset(&b, 0, sizeof(b));
-            for (int f = 0; f < 6; ++f) {
-                if (!on[f]) continue;
-                const FieldGeom g = geom(c, f);
-                GemmProb& p = b.p[b.count++];
-                switch (stage) {
-                    case 0:   // t1 = X R
-                        p.A = c->rhs[f] + g.off; p.lda = N;
-                        p.B = g.R; p.ldb = g.ldR;
-                        p.C = c->t1[f]; p.ldc = N;
-                        p.M = g.rows; p.N = g.cols; p.K = g.cols;
-                        break;
-                    case 1:   // t2 = Lambda o (L t1)
-                        p.A = g.L; p.lda = g.ldL;
-                        p.B = c->t1[f]; p.ldb = N;
-                        p.C = c->t2[f]; p.ldc = N;
-                        p.L = g.Lam; p.ldl = g.ldLam;
-                        p.M = g.rows; p.N = g.cols; p.K = g.rows;
-                        break;
-                    case 2:   // t1 = t2 R
-                        p.A = c->t2[f]; p.lda = N;
-                        p.B = g.R; p.ldb = g.ldR;
-                        p.C = c->t1[f]; p.ldc = N;
-                        p.M = g.rows; p.N = g.cols; p.K = g.cols;
-                        break;
-                    default:  // out = L t1
-                        p.A = g.L; p.lda = g.ldL;
-                        p.B = c->t1[f]; p.ldb = N;
-                        p.C = dst[f] + g.off; p.ldc = N;
-                        p.M = g.rows; p.N = g.cols; p.K = g.rows;
-                        break;
-                }
-            }
-            LC3D_TRY(launch_gemm(c, b, s));
+        DenseDesc d[6]{};
+        int cnt = 0;
+        for (int f = 0; f < 6; ++f) {
+            if (!on[f]) continue;
+            const FieldGeom g = geom(c, f);
+            d[cnt++] = {c->rhs[f] + g.off, g.type0, g.type1, c->t1[f], c->t2[f], dst[f] + g.off};
         }
+        LC3D_TRY(dense_solve(c, d, cnt, s));
     }
     const double inv_n = 1.0 / n;
     if (on[5] && !bz_partials) {

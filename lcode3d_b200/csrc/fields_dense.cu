@@ -1,0 +1,372 @@
+// Spectral field solves in dense-transform (GEMM) form, float64: grids whose
+// 2 (N - 1) has other factors than 2, 3 and 5, and lc3d_fp64_transform =
+// 'dense'.
+//
+// A solve is F = L (Lambda o (L X R)) R with the DST-I / DCT-I matrices of
+// fields.cu. Rows of T = S2 or C are even or odd about their centre c,
+//     T[k][m - n] = (-1)^k T[k][n],   m the last index,
+// so along each axis the even outputs see only x[n] + x[m - n] and the odd
+// ones x[n] - x[m - n]: two transforms of half the size, half the products.
+// A solve folds X once along both axes (even part first, then odd, in rows
+// and in columns), keeps the spectrum sorted by parity (Lambda to match) and
+// unfolds once at the end:
+//     fold, t1 = X R, t2 = Lambda o (L t1), t1 = t2 R', t2 = L' t1, unfold
+// with L, R block diagonal in the parity: 12 GEMMs (6 fields, 2 parities) per
+// launch. (' : the matrices of the way back, F[n] = sum_k T[n][k] G[k].)
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "lc3d_internal.cuh"
+
+namespace {
+
+// ---------------------------------------------------------------------------
+// Fold and unfold
+// ---------------------------------------------------------------------------
+struct FoldArgs {
+    const double* in[6];
+    double* out[6];
+    int ld_in, ld_out;
+    int rows[6], cols[6];
+};
+
+// One thread per (a, b), a <= (rows - 1) / 2, b <= (cols - 1) / 2 (sizes are
+// odd): the four cells it mirrors to, and the four sums and differences. The
+// centre is its own mirror and belongs to the even part alone.
+__global__ void __launch_bounds__(128) fold_kernel(const __grid_constant__ FoldArgs g) {
+    pdl_wait();
+    const int f = blockIdx.z, a = blockIdx.y, b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c0 = (g.rows[f] - 1) / 2, c1 = (g.cols[f] - 1) / 2;
+    if (a > c0 || b > c1) return;
+    const int a2 = g.rows[f] - 1 - a, b2 = g.cols[f] - 1 - b;
+    const double* x = g.in[f];
+    const double x00 = x[(size_t)a * g.ld_in + b];
+    const double x01 = b < c1 ? x[(size_t)a * g.ld_in + b2] : 0.0;
+    const double x10 = a < c0 ? x[(size_t)a2 * g.ld_in + b] : 0.0;
+    const double x11 = a < c0 && b < c1 ? x[(size_t)a2 * g.ld_in + b2] : 0.0;
+    double* o = g.out[f];
+    const size_t even = (size_t)a * g.ld_out, odd = (size_t)(c0 + 1 + a) * g.ld_out;
+    o[even + b] = (x00 + x01) + (x10 + x11);
+    if (b < c1) o[even + c1 + 1 + b] = (x00 - x01) + (x10 - x11);
+    if (a < c0) o[odd + b] = (x00 + x01) - (x10 + x11);
+    if (a < c0 && b < c1) o[odd + c1 + 1 + b] = (x00 - x01) - (x10 - x11);
+}
+
+// The inverse walk: value and mirrors from the even and odd parts.
+__global__ void __launch_bounds__(128) unfold_kernel(const __grid_constant__ FoldArgs g) {
+    pdl_wait();
+    const int f = blockIdx.z, a = blockIdx.y, b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c0 = (g.rows[f] - 1) / 2, c1 = (g.cols[f] - 1) / 2;
+    if (a > c0 || b > c1) return;
+    const int a2 = g.rows[f] - 1 - a, b2 = g.cols[f] - 1 - b;
+    const double* x = g.in[f];
+    const size_t even = (size_t)a * g.ld_in, odd = (size_t)(c0 + 1 + a) * g.ld_in;
+    const double ee = x[even + b];
+    const double eo = b < c1 ? x[even + c1 + 1 + b] : 0.0;
+    const double oe = a < c0 ? x[odd + b] : 0.0;
+    const double oo = a < c0 && b < c1 ? x[odd + c1 + 1 + b] : 0.0;
+    double* o = g.out[f];
+    o[(size_t)a * g.ld_out + b] = (ee + eo) + (oe + oo);
+    if (b < c1) o[(size_t)a * g.ld_out + b2] = (ee - eo) + (oe - oo);
+    if (a < c0) o[(size_t)a2 * g.ld_out + b] = (ee + eo) - (oe + oo);
+    if (a < c0 && b < c1) o[(size_t)a2 * g.ld_out + b2] = (ee - eo) - (oe - oo);
+}
+
+// out[i][j] = lam[k0 of i][k1 of j], both axes sorted by parity.
+__global__ void lam_parity_kernel(const double* __restrict__ lam, int rows, int cols, double* __restrict__ out) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+    if (j >= cols) return;
+    const int e0 = (rows + 1) / 2, e1 = (cols + 1) / 2;
+    const int k0 = i < e0 ? 2 * i : 2 * (i - e0) + 1, k1 = j < e1 ? 2 * j : 2 * (j - e1) + 1;
+    out[(size_t)i * cols + j] = lam[(size_t)k0 * cols + k1];
+}
+
+// ---------------------------------------------------------------------------
+// Batched float64 GEMM, C = A B (optionally C = Lambda o (A B)), row-major,
+// on the float64 tensor cores (mma.sync m8n8k4 .f64: each product and sum is
+// an IEEE float64 fused multiply-add). 64 x 32 tiles per 64-thread CTA, a
+// 32 x 32 tile (4 x 4 MMAs per k4 step) per warp; k-steps of 16 staged by
+// cp.async into two shared-memory buffers, the next k-step copied while the
+// current one is multiplied.
+//
+// The tile is small because the problems are: at 387^2 a launch has 12 of
+// about 387 x 194 x 194, and what is lost is rows and columns past the edges
+// and SMs with a tile less than others. GEMM_FIGURES
+// ---------------------------------------------------------------------------
+constexpr int MAX_PROBS = 12;
+
+struct GemmProb {
+    const double *A, *B, *L;
+    double* C;
+    int M, N, K, lda, ldb, ldc, ldl;
+    int tiles_n, tile_start;
+};
+
+struct GemmBatch {
+    GemmProb p[MAX_PROBS];
+    int count;
+};
+
+constexpr int GTM = 64, GTN = 32, GK = 16;
+constexpr int GEMM_THREADS = GTM / 32 * (GTN / 32) * 32;
+// shared pitches (doubles): the fragment loads of a half-warp (rows g = 0..3
+// or 4..7, columns t = 0..3) fall in distinct banks: 2 (20 g + t) and
+// 2 (36 t + g) mod 32 are distinct over the 16 lanes
+constexpr int AS_LD = GK + 4;    // As[m][k]
+constexpr int BS_LD = GTN + 4;   // Bs[k][n]
+constexpr int AS_SIZE = GTM * AS_LD, BS_SIZE = GK * BS_LD;
+
+// 8-byte global -> shared copy; a source size of 0 writes zeros (the tile
+// edges past M, N or K).
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool in) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(in ? 8 : 0) : "memory");
+}
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+__global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_constant__ GemmBatch b) {
+    __shared__ __align__(16) double As[2 * AS_SIZE], Bs[2 * BS_SIZE];
+    const int bid = blockIdx.x;
+    int pi = 0;
+#pragma unroll 1
+    for (int q = 1; q < b.count; ++q)
+        if (bid >= b.p[q].tile_start) pi = q;
+    const GemmProb& P = b.p[pi];
+    const int t = bid - P.tile_start;
+    const int tm = t / P.tiles_n, tn = t - tm * P.tiles_n;
+    const int row0 = tm * GTM, col0 = tn * GTN;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, tq = lane & 3;            // fragment row group, thread in group
+    const int wm = warp % (GTM / 32) * 32, wn = warp / (GTM / 32) * 32;
+    pdl_wait();
+
+    auto load = [&](int k0, int buf) {
+        double* as = As + buf * AS_SIZE;
+        double* bs = Bs + buf * BS_SIZE;
+#pragma unroll
+        for (int i = 0; i < GTM * GK / GEMM_THREADS; ++i) {   // rows idx / 16, k idx % 16
+            const int idx = tid + i * GEMM_THREADS, r = idx / GK, kk = idx % GK;
+            const int row = row0 + r, k = k0 + kk;
+            const bool in = row < P.M && k < P.K;
+            cp_async8(as + r * AS_LD + kk, in ? P.A + (size_t)row * P.lda + k : P.A, in);
+        }
+#pragma unroll
+        for (int i = 0; i < GK * GTN / GEMM_THREADS; ++i) {   // k rows idx / GTN, columns idx % GTN
+            const int idx = tid + i * GEMM_THREADS, kk = idx / GTN, n = idx % GTN;
+            const int k = k0 + kk, col = col0 + n;
+            const bool in = k < P.K && col < P.N;
+            cp_async8(bs + kk * BS_LD + n, in ? P.B + (size_t)k * P.ldb + col : P.B, in);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    double acc[4][4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+
+    const int nk = (P.K + GK - 1) / GK;
+    load(0, 0);
+    for (int kt = 0; kt < nk; ++kt) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();   // k-step kt is in; every warp is done with the other buffer
+        if (kt + 1 < nk) load((kt + 1) * GK, (kt + 1) & 1);
+        const double* as = As + (kt & 1) * AS_SIZE + (wm + g) * AS_LD + tq;
+        const double* bs = Bs + (kt & 1) * BS_SIZE + tq * BS_LD + wn + g;
+#pragma unroll
+        for (int ks = 0; ks < GK; ks += 4) {
+            double af[4], bf[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) af[i] = as[i * 8 * AS_LD + ks];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) bf[j] = bs[ks * BS_LD + j * 8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dmma(acc[i][j], af[i], bf[j]);
+        }
+    }
+    // accumulator (i, j, h): row wm + 8 i + g, column wn + 8 j + 2 tq + h
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int row = row0 + wm + 8 * i + g;
+        if (row >= P.M) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int col = col0 + wn + 8 * j + 2 * tq + h;
+                if (col >= P.N) continue;
+                double v = acc[i][j][h];
+                if (P.L) v *= P.L[(size_t)row * P.ldl + col];
+                P.C[(size_t)row * P.ldc + col] = v;
+            }
+        }
+    }
+}
+
+int launch_gemm(lc3d_ctx* c, GemmBatch& b, cudaStream_t s) {
+    int tiles = 0;
+    for (int q = 0; q < b.count; ++q) {
+        GemmProb& p = b.p[q];
+        p.tiles_n = (p.N + GTN - 1) / GTN;
+        p.tile_start = tiles;
+        tiles += ((p.M + GTM - 1) / GTM) * p.tiles_n;
+    }
+    if (tiles == 0) return LC3D_OK;
+    ProfScope ps(c, LC3D_STAGE_TRANSFORM, s);
+    LC3D_CUDA_TRY(launch_pdl(dgemm_kernel, dim3(tiles), dim3(GEMM_THREADS), 0, s, b));
+    LC3D_CUDA_TRY(cudaGetLastError());
+    return LC3D_OK;
+}
+
+// sin(pi r / L) for integer r, with the argument reduced to [0, pi/2].
+double sin_pi_frac(long long r, long long L) {
+    r %= 2 * L;
+    if (r < 0) r += 2 * L;
+    double sign = 1;
+    if (r >= L) { r -= L; sign = -1; }
+    if (2 * r > L) r = L - r;
+    return sign * std::sin(M_PI * (double)r / (double)L);
+}
+
+// Half-size matrices of a transform type, by parity q (0 even, 1 odd) of the
+// frequency: forth[k][n] = T[2 k + q][n], back[n][k] = T[n][2 k + q], and
+// their transposes, all n_q x n_q.
+struct HalfMats {
+    double *forth, *forth_t, *back, *back_t;
+};
+
+struct DenseState {
+    HalfMats m[2][2];       // [type][parity]
+    double* lam[4];         // by type0 * 2 + type1, sorted by parity
+};
+
+// Size of parity q's half of a transform of `n` points (odd).
+int half(int n, int q) { return q ? n / 2 : n / 2 + 1; }
+
+}  // namespace
+
+int dense_init(lc3d_ctx* c) {
+    DenseState* d = new DenseState();
+    c->dense = d;
+    const int N = c->N;
+    const long long L = N - 1;
+    for (int type = 0; type < 2; ++type)
+        for (int q = 0; q < 2; ++q) {
+            const int n = half(N - 2 * type, q);
+            // T[k][x]: 2 sin(pi (k+1)(x+1) / L), or c_x cos(pi k x / L) with
+            // cos(pi r / L) = sin(pi (2 r + L) / (2 L))
+            auto T = [&](long long k, long long x) {
+                if (type) return 2 * sin_pi_frac((k + 1) * (x + 1), L);
+                const long long r = (k * x) % (2 * L);
+                return (x == 0 || x == L ? 1.0 : 2.0) * sin_pi_frac(2 * r + L, 2 * L);
+            };
+            const size_t nn = (size_t)n * n;
+            std::vector<double> h(4 * nn);
+            for (int k = 0; k < n; ++k)
+                for (int x = 0; x < n; ++x) {
+                    const double f = T(2 * k + q, x), b = T(x, 2 * k + q);
+                    h[(size_t)k * n + x] = f;
+                    h[nn + (size_t)x * n + k] = f;
+                    h[2 * nn + (size_t)x * n + k] = b;
+                    h[3 * nn + (size_t)k * n + x] = b;
+                }
+            HalfMats& m = d->m[type][q];
+            LC3D_CUDA_TRY(cudaMalloc(&m.forth, 4 * nn * sizeof(double)));
+            LC3D_CUDA_TRY(cudaMemcpy(m.forth, h.data(), 4 * nn * sizeof(double), cudaMemcpyHostToDevice));
+            m.forth_t = m.forth + nn;
+            m.back = m.forth + 2 * nn;
+            m.back_t = m.forth + 3 * nn;
+        }
+    const double* src[4] = {c->lam_neu, c->lam_mixT, c->lam_mix, c->lam_dir};
+    for (int k = 0; k < 4; ++k) {
+        const int rows = N - 2 * (k >> 1), cols = N - 2 * (k & 1);
+        LC3D_CUDA_TRY(cudaMalloc(&d->lam[k], (size_t)rows * cols * sizeof(double)));
+        lam_parity_kernel<<<dim3((cols + 127) / 128, rows), 128>>>(src[k], rows, cols, d->lam[k]);
+        LC3D_CUDA_TRY(cudaGetLastError());
+    }
+    return LC3D_OK;
+}
+
+void dense_free(lc3d_ctx* c) {
+    DenseState* d = static_cast<DenseState*>(c->dense);
+    if (!d) return;
+    for (auto& type : d->m)
+        for (HalfMats& m : type)
+            if (m.forth) cudaFree(m.forth);
+    for (double* l : d->lam)
+        if (l) cudaFree(l);
+    delete d;
+    c->dense = nullptr;
+}
+
+int dense_solve(lc3d_ctx* c, const DenseDesc* desc, int count, cudaStream_t s) {
+    const DenseState* d = static_cast<const DenseState*>(c->dense);
+    const int N = c->N;
+    const dim3 fold_grid(((N + 1) / 2 + 127) / 128, (N + 1) / 2, count);
+    FoldArgs fa{};
+    fa.ld_in = fa.ld_out = N;
+    for (int f = 0; f < count; ++f) {
+        fa.rows[f] = N - 2 * desc[f].type0;
+        fa.cols[f] = N - 2 * desc[f].type1;
+        fa.in[f] = desc[f].rhs;
+        fa.out[f] = desc[f].t2;
+    }
+    {
+        ProfScope ps(c, LC3D_STAGE_TRANSFORM, s);
+        LC3D_CUDA_TRY(launch_pdl(fold_kernel, fold_grid, dim3(128), 0, s, fa));
+        LC3D_CUDA_TRY(cudaGetLastError());
+    }
+    for (int stage = 0; stage < 4; ++stage) {
+        GemmBatch b;
+        memset(&b, 0, sizeof(b));
+        for (int f = 0; f < count; ++f) {
+            const DenseDesc& e = desc[f];
+            const int rows = fa.rows[f], cols = fa.cols[f];
+            const bool right = stage == 0 || stage == 2, back = stage >= 2;
+            for (int q = 0; q < 2; ++q) {
+                GemmProb& p = b.p[b.count++];
+                const double* in = right ? e.t2 : e.t1;
+                double* out = right ? e.t1 : e.t2;
+                if (right) {        // columns of parity q
+                    const int n = half(cols, q), at = q * half(cols, 0);
+                    const HalfMats& m = d->m[e.type1][q];
+                    p.A = in + at; p.lda = N;
+                    p.B = back ? m.back_t : m.forth_t; p.ldb = n;
+                    p.C = out + at; p.ldc = N;
+                    p.M = rows; p.N = n; p.K = n;
+                } else {            // rows of parity q
+                    const int n = half(rows, q), at = q * half(rows, 0);
+                    const HalfMats& m = d->m[e.type0][q];
+                    p.A = back ? m.back : m.forth; p.lda = n;
+                    p.B = in + (size_t)at * N; p.ldb = N;
+                    p.C = out + (size_t)at * N; p.ldc = N;
+                    p.M = n; p.N = cols; p.K = n;
+                    if (!back) {
+                        p.L = d->lam[e.type0 * 2 + e.type1] + (size_t)at * cols;
+                        p.ldl = cols;
+                    }
+                }
+            }
+        }
+        LC3D_TRY(launch_gemm(c, b, s));
+    }
+    for (int f = 0; f < count; ++f) {
+        fa.in[f] = desc[f].t2;
+        fa.out[f] = desc[f].out;
+    }
+    ProfScope ps(c, LC3D_STAGE_TRANSFORM, s);
+    LC3D_CUDA_TRY(launch_pdl(unfold_kernel, fold_grid, dim3(128), 0, s, fa));
+    LC3D_CUDA_TRY(cudaGetLastError());
+    return LC3D_OK;
+}

@@ -216,6 +216,18 @@ void fft64_free(lc3d_ctx* ctx);
 int fft64_pitch(int N);
 int fft64_solve(lc3d_ctx* ctx, const Fft64Desc* desc, int count, cudaStream_t s);
 
+// Float64 dense solves (fields_dense.cu): the right-hand sides of `count` fields
+// to their raw solutions, both inside N x N planes (row pitch N).
+struct DenseDesc {
+    const double* rhs;                    // (N - 2 type0) x (N - 2 type1)
+    int type0, type1;                     // axis-0 / axis-1 transform: 0 DCT-I, 1 DST-I
+    double *t1, *t2;                      // intermediates
+    double* out;
+};
+int dense_init(lc3d_ctx* ctx);
+void dense_free(lc3d_ctx* ctx);
+int dense_solve(lc3d_ctx* ctx, const DenseDesc* desc, int count, cudaStream_t s);
+
 // Mixed-precision transform stages (fields_mixed.cu): C = A B^T with one
 // operand a sliced fixed transform matrix (0 = S2, 1 = C) and the other the
 // float64 data operand `data` (data_rows x K, row-major, ld_data), sliced
@@ -278,7 +290,6 @@ struct lc3d_ctx {
     cudaStream_t fft_stream[2];           // further streams of the FFT passes (groups of fields)
     cudaEvent_t ev_fork, ev_join[2];      // their fork from and joins to the solve's stream
     // field-solver workspaces (fields.cu)
-    double *S2, *C, *CT;                  // 2*DST-I (M x M), DCT-I (N x N), its transpose
     double *lam_dir, *lam_mix, *lam_mixT, *lam_neu;
     float *lam32_dir, *lam32_mix, *lam32_mixT, *lam32_neu;   // float32-transform precision only
     double* rhs[6];                       // right-hand sides, N x N planes
@@ -292,6 +303,7 @@ struct lc3d_ctx {
     int fft_grid[3];                      // persistent FFT grid per FftTypes instantiation
     int fft_sms;                          // SMs of the device (the grid cap of lc3d_set_tiles)
     void* fft64;                          // float64 FFT solves (fields_fft64.cu)
+    void* dense;                          // float64 dense solves (fields_dense.cu)
     void* mixed;                          // mixed-precision solver state (fields_mixed.cu)
     // launch accounting / profiling
     long long launches[LC3D_NSTAGES];

@@ -86,15 +86,18 @@ __global__ void lam_parity_kernel(const double* __restrict__ lam, int rows, int 
 
 // ---------------------------------------------------------------------------
 // Batched float64 GEMM, C = A B (optionally C = Lambda o (A B)), row-major,
-// on the float64 tensor cores (mma.sync m8n8k4 .f64: each product and sum is
-// an IEEE float64 fused multiply-add). 64 x 32 tiles per 64-thread CTA, a
-// 32 x 32 tile (4 x 4 MMAs per k4 step) per warp; k-steps of 16 staged by
+// on the float64 tensor cores (mma.sync m16n8k8 .f64: float64 products and
+// sums throughout). 64 x 32 tiles per 64-thread CTA, a 32 x 32 tile (2 x 4
+// MMAs per k8 step) per warp; k-steps of 16 staged by
 // cp.async into two shared-memory buffers, the next k-step copied while the
 // current one is multiplied.
 //
 // The tile is small because the problems are: at 387^2 a launch has 12 of
 // about 387 x 194 x 194, and what is lost is rows and columns past the edges
-// and SMs with a tile less than others. GEMM_FIGURES
+// and SMs with a tile less than others. 28 us a launch at 387^2 (two or three
+// 64 x 32 tiles' k-steps in flight per scheduler; 35 with m8n8k4 MMAs and
+// bounds checks on every copy); 78 with matrices of full size in 128 x 64
+// tiles.
 // ---------------------------------------------------------------------------
 constexpr int MAX_PROBS = 12;
 
@@ -119,17 +122,19 @@ constexpr int AS_LD = GK + 4;    // As[m][k]
 constexpr int BS_LD = GTN + 4;   // Bs[k][n]
 constexpr int AS_SIZE = GTM * AS_LD, BS_SIZE = GK * BS_LD;
 
-// 8-byte global -> shared copy; a source size of 0 writes zeros (the tile
-// edges past M, N or K).
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool in) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(in ? 8 : 0) : "memory");
+// 8-byte global -> shared copy; a source size of 0 writes zeros.
+__device__ __forceinline__ void cp_async8(uint32_t dst, const double* src, int size) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
 }
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
+// c += a b, 16 x 8 x 8. Thread (g, t) = (lane / 4, lane % 4) holds a[i] at
+// row g + 8 (i & 1), k t + 4 (i >> 1); b[i] at k t + 4 i, column g; c[i] at
+// row g + 8 (i >> 1), column 2 t + (i & 1).
+__device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
 __global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_constant__ GemmBatch b) {
@@ -148,31 +153,40 @@ __global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_con
     const int wm = warp % (GTM / 32) * 32, wn = warp / (GTM / 32) * 32;
     pdl_wait();
 
+    // Rows of A past M and columns of B past N repeat the last one (nothing of
+    // them is stored), so a copy's address costs a clamp and a multiply; past
+    // K zeros are copied. A: 4 rows x 16 k per pass of the threads; B: 2 k
+    // rows x 32 columns.
+    static_assert(GEMM_THREADS == 64 && GK == 16 && GTN == 32, "the copies' shapes");
+    const int ra = tid / GK, ka = tid % GK, kb = tid / GTN, nb = tid % GTN;
+    const int alast = P.M - 1 - row0 - ra, astep = 4;
+    const double* pa = P.A + (size_t)(row0 + ra) * P.lda + ka;
+    const double* pb = P.B + (size_t)kb * P.ldb + min(col0 + nb, P.N - 1);
+    const uint32_t sa = static_cast<uint32_t>(__cvta_generic_to_shared(As + ra * AS_LD + ka));
+    const uint32_t sb = static_cast<uint32_t>(__cvta_generic_to_shared(Bs + kb * BS_LD + nb));
     auto load = [&](int k0, int buf) {
-        double* as = As + buf * AS_SIZE;
-        double* bs = Bs + buf * BS_SIZE;
+        const int size_a = k0 + ka < P.K ? 8 : 0;
+        const double* a = size_a ? pa + k0 : P.A;
+        const int lda = size_a ? P.lda : 0;
 #pragma unroll
-        for (int i = 0; i < GTM * GK / GEMM_THREADS; ++i) {   // rows idx / 16, k idx % 16
-            const int idx = tid + i * GEMM_THREADS, r = idx / GK, kk = idx % GK;
-            const int row = row0 + r, k = k0 + kk;
-            const bool in = row < P.M && k < P.K;
-            cp_async8(as + r * AS_LD + kk, in ? P.A + (size_t)row * P.lda + k : P.A, in);
-        }
+        for (int i = 0; i < GTM / astep; ++i)
+            cp_async8(sa + (buf * AS_SIZE + i * astep * AS_LD) * 8, a + (ptrdiff_t)min(i * astep, alast) * lda, size_a);
+        const double* b = pb + (size_t)k0 * P.ldb;
 #pragma unroll
-        for (int i = 0; i < GK * GTN / GEMM_THREADS; ++i) {   // k rows idx / GTN, columns idx % GTN
-            const int idx = tid + i * GEMM_THREADS, kk = idx / GTN, n = idx % GTN;
-            const int k = k0 + kk, col = col0 + n;
-            const bool in = k < P.K && col < P.N;
-            cp_async8(bs + kk * BS_LD + n, in ? P.B + (size_t)k * P.ldb + col : P.B, in);
+        for (int i = 0; i < GK / 2; ++i) {
+            const bool in = k0 + kb + 2 * i < P.K;
+            cp_async8(sb + (buf * BS_SIZE + i * 2 * BS_LD) * 8, in ? b + (ptrdiff_t)(2 * i) * P.ldb : P.B, in ? 8 : 0);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    double acc[4][4][2];
+    double acc[2][4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) acc[i][j][h] = 0.0;
 
     const int nk = (P.K + GK - 1) / GK;
     load(0, 0);
@@ -183,33 +197,42 @@ __global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_con
         const double* as = As + (kt & 1) * AS_SIZE + (wm + g) * AS_LD + tq;
         const double* bs = Bs + (kt & 1) * BS_SIZE + tq * BS_LD + wn + g;
 #pragma unroll
-        for (int ks = 0; ks < GK; ks += 4) {
-            double af[4], bf[4];
+        for (int ks = 0; ks < GK; ks += 8) {
+            double af[2][4], bf[4][2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) af[i] = as[i * 8 * AS_LD + ks];
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) bf[j] = bs[ks * BS_LD + j * 8];
+                for (int h = 0; h < 4; ++h) af[i][h] = as[(i * 16 + (h & 1) * 8) * AS_LD + ks + (h >> 1) * 4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) bf[j][h] = bs[(ks + h * 4) * BS_LD + j * 8];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) dmma(acc[i][j], af[i], bf[j]);
         }
     }
-    // accumulator (i, j, h): row wm + 8 i + g, column wn + 8 j + 2 tq + h
+    // accumulator (i, j, h): row wm + 16 i + g + 8 (h >> 1), column wn + 8 j +
+    // 2 tq + (h & 1); a row's Lambda values are loaded together, ahead of its stores
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int row = row0 + wm + 8 * i + g;
+        const int row = row0 + wm + 8 * i + g, c0 = col0 + wn + 2 * tq;
         if (row >= P.M) continue;
+        double l[8];
+        if (P.L)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int col = col0 + wn + 8 * j + 2 * tq + h;
-                if (col >= P.N) continue;
-                double v = acc[i][j][h];
-                if (P.L) v *= P.L[(size_t)row * P.ldl + col];
-                P.C[(size_t)row * P.ldc + col] = v;
+            for (int u = 0; u < 8; ++u) {
+                const int col = c0 + u / 2 * 8 + u % 2;
+                l[u] = col < P.N ? __ldg(P.L + (size_t)row * P.ldl + col) : 0.0;
             }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int col = c0 + u / 2 * 8 + u % 2;
+            if (col >= P.N) continue;
+            double v = acc[i >> 1][u / 2][(i & 1) * 2 + u % 2];
+            if (P.L) v *= l[u];
+            P.C[(size_t)row * P.ldc + col] = v;
         }
     }
 }

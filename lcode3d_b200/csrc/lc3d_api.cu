@@ -132,14 +132,14 @@ MoveArgs move_base(lc3d_ctx* c) {
     return a;
 }
 
-DepositArgs deposit_args(lc3d_ctx* c, const double* x, const double* y, const double* m, const double* q,
+DepositArgs deposit_args(lc3d_ctx* c, int buf, const double* x, const double* y, const double* m, const double* q,
                          const double* px, const double* py, const double* pz, const double* packed) {
     DepositArgs a{};
     a.x_offt = x; a.y_offt = y; a.m = m; a.q = q; a.px = px; a.py = py; a.pz = pz;
     a.packed = packed;   // the same values, packed by the move just before
     a.inf_prev = c->inf_prev; a.inf_next = c->inf_next; a.fine_grid = c->fine_grid;
     a.idx_prev = c->idx_prev; a.idx_next = c->idx_next;
-    a.acc = c->acc;
+    a.acc = c->acc[buf];
     a.plane = c->acc_plane;
     a.Nc = c->Nc; a.Nf = c->Nf; a.N = c->N;
     a.fine_off = deposit_fine_offset(c->p.plasma_fineness);
@@ -152,7 +152,7 @@ DepositArgs deposit_args(lc3d_ctx* c, const double* x, const double* y, const do
 DepositFinalizeArgs finalize_args(lc3d_ctx* c, const double* ro_initial, double* ro, double* jx, double* jy,
                                   double* jz) {
     DepositFinalizeArgs f{};
-    f.acc = c->acc;
+    f.acc = c->acc[0];
     f.plane = c->acc_plane;
     f.ro_initial = ro_initial;
     f.ro = ro; f.jx = jx; f.jy = jy; f.jz = jz;
@@ -163,7 +163,7 @@ DepositFinalizeArgs finalize_args(lc3d_ctx* c, const double* ro_initial, double*
 int deposit_into(lc3d_ctx* c, const double* ro_initial, const double* x, const double* y, const double* m,
                  const double* q, const double* px, const double* py, const double* pz, double* ro, double* jx,
                  double* jy, double* jz, cudaStream_t s, const double* packed = nullptr) {
-    const DepositArgs a = deposit_args(c, x, y, m, q, px, py, pz, packed);
+    const DepositArgs a = deposit_args(c, 0, x, y, m, q, px, py, pz, packed);
     const DepositFinalizeArgs f = finalize_args(c, ro_initial, ro, jx, jy, jz);
     {
         ProfScope ps(c, LC3D_STAGE_DEPOSIT, s);
@@ -171,6 +171,24 @@ int deposit_into(lc3d_ctx* c, const double* ro_initial, const double* x, const d
     }
     ProfScope ps(c, LC3D_STAGE_DEPOSIT_FIN, s);
     return launch_deposit_finalize(f, s);
+}
+
+// A deposition that ends in the accumulators `buf`, for a solve that reads them.
+int deposit_raw(lc3d_ctx* c, int buf, double* const* pw, cudaStream_t s) {
+    ProfScope ps(c, LC3D_STAGE_DEPOSIT, s);
+    return launch_deposit_main(deposit_args(c, buf, pw[0], pw[1], c->m, c->q, pw[2], pw[3], pw[4], c->packed), s);
+}
+
+// The accumulators of pass `pass` (0 predictor, 1 corrector) as a solve's
+// densities. Each pass has its own, and its solve clears the other's: reading
+// and clearing the same cells in one kernel would race on the neighbours the
+// right-hand sides read. accumulators 0 are clear between steps (the final
+// deposition uses them and its finalize clears them); 1 hold the last
+// corrector's until the next predictor's solve.
+void solve_from_acc(lc3d_ctx* c, int pass, SolveInputs& in) {
+    in.acc = c->acc[pass];
+    in.acc_clear = c->acc[pass ^ 1];
+    in.ro_initial = c->ro_initial;
 }
 
 // Optional extras of a step: first-pass fields out, or a prediction that
@@ -297,8 +315,13 @@ int run_step(lc3d_ctx* c, const lc3d_state_ptrs& prev, const lc3d_state_ptrs& ou
             LC3D_CUDA_TRY(cudaGetLastError());
             continue;
         }
-        LC3D_TRY(deposit_into(c, c->ro_initial, pw[0], pw[1], c->m, c->q, pw[2], pw[3], pw[4], c->dens[0],
-                              c->dens[1], c->dens[2], c->dens[3], s, c->packed));
+        if (predicted) {   // no predictor solve: accumulators 1 are not clear
+            LC3D_TRY(deposit_into(c, c->ro_initial, pw[0], pw[1], c->m, c->q, pw[2], pw[3], pw[4], c->dens[0],
+                                  c->dens[1], c->dens[2], c->dens[3], s, c->packed));
+        } else {
+            LC3D_TRY(deposit_raw(c, pass, pw, s));
+            solve_from_acc(c, pass, in);
+        }
         if (pass == 0) {
             in.Ex_sub = prev.Ex; in.Ey_sub = prev.Ey; in.Bx_sub = prev.Bx; in.By_sub = prev.By;
             for (int f = 0; f < 6; ++f) so.out[f] = (x && x->first) ? x->first[f] : nullptr;
@@ -356,7 +379,8 @@ void destroy(lc3d_ctx* c) {
         if (c->dens[k]) cudaFree(c->dens[k]);
     for (int k = 0; k < 6; ++k)
         if (c->avg[k]) cudaFree(c->avg[k]);
-    if (c->acc) cudaFree(c->acc);
+    for (int a = 0; a < 2; ++a)
+        if (c->acc[a]) cudaFree(c->acc[a]);
     if (c->err) cudaFree(c->err);
     if (c->err_host) cudaFreeHost(c->err_host);
     if (c->zeros) cudaFree(c->zeros);
@@ -465,8 +489,9 @@ int step_schedule(lc3d_ctx* c, const lc3d_state_ptrs& prev, const lc3d_state_ptr
 // whose depositions run as one launch over all simulations. Segment `seg`
 // enqueues the launches between deposition seg - 1 and deposition seg and
 // returns the kernel arguments of deposition seg in *dep (segments 0-2);
-// the finalize of deposition seg - 1 opens segment seg (1-3). The launches
-// and their order are those of run_step without extras.
+// the solve of deposition seg - 1 opens segment 1 or 2, the last one's
+// finalize segment 3. The launches and their order are those of run_step
+// without extras.
 int step_schedule_segment(lc3d_ctx* c, const lc3d_state_ptrs& prev, const lc3d_state_ptrs& out,
                           const double* beam, cudaStream_t s, int seg, DepositArgs* dep) {
     const double* prevF[6] = {prev.Ex, prev.Ey, prev.Ez, prev.Bx, prev.By, prev.Bz};
@@ -489,7 +514,7 @@ int step_schedule_segment(lc3d_ctx* c, const lc3d_state_ptrs& prev, const lc3d_s
         mv.out_px = o ? o[2] : out.px; mv.out_py = o ? o[3] : out.py; mv.out_pz = o ? o[4] : out.pz;
         ProfScope ps(c, LC3D_STAGE_MOVE, s);
         LC3D_TRY(launch_move_smart(mv, s));
-        *dep = deposit_args(c, mv.out_x, mv.out_y, c->m, c->q, mv.out_px, mv.out_py, mv.out_pz, c->packed);
+        *dep = deposit_args(c, pass & 1, mv.out_x, mv.out_y, c->m, c->q, mv.out_px, mv.out_py, mv.out_pz, c->packed);
         return LC3D_OK;
     };
     auto finalize = [&](double* ro, double* jx, double* jy, double* jz) -> int {
@@ -500,9 +525,8 @@ int step_schedule_segment(lc3d_ctx* c, const lc3d_state_ptrs& prev, const lc3d_s
     if (seg == 3) return finalize(out.ro, out.jx, out.jy, out.jz);
     if (seg != 1 && seg != 2) return LC3D_ERR_PARAM;
     const int pass = seg - 1;
-    LC3D_TRY(finalize(c->dens[0], c->dens[1], c->dens[2], c->dens[3]));
     SolveInputs in{};
-    in.ro = c->dens[0]; in.jx = c->dens[1]; in.jy = c->dens[2]; in.jz = c->dens[3];
+    solve_from_acc(c, pass, in);
     in.ro_prev = A ? prev.ro : nullptr;
     in.jz_prev = A ? prev.jz : nullptr;
     in.jx_prev = prev.jx; in.jy_prev = prev.jy;
@@ -587,7 +611,7 @@ int lc3d_create(const lc3d_params* p, int device, lc3d_ctx** out) {
     for (int k = 0; k < 4; ++k) LC3D_STEP(dalloc(&c->dens[k], ng));
     for (int k = 0; k < 6; ++k) LC3D_STEP(dalloc(&c->avg[k], ng));
     c->acc_plane = (ng + 31) / 32 * 32;
-    LC3D_STEP(dalloc(&c->acc, c->acc_plane * 8));
+    for (int a = 0; a < 2; ++a) LC3D_STEP(dalloc(&c->acc[a], c->acc_plane * DEP_WORDS_PER_CELL));
     LC3D_STEP(dalloc(&c->err, (size_t)1));
     // pinned host word the flag is read into (a direct copy, no staging)
     if (rc == LC3D_OK && cudaHostAlloc(&c->err_host, sizeof(unsigned), cudaHostAllocDefault) != cudaSuccess)

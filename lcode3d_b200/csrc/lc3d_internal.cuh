@@ -112,6 +112,13 @@ struct DepositFinalizeArgs {
     int vec;                              // set by the launcher: 16-byte aligned float64 arrays
 };
 
+// The deposition's accumulators: planes of 64-bit words, hi and lo of ro, jx,
+// jy, jz in turn; a density is hi 2^-24 + lo 2^-76.
+constexpr int DEP_WORDS_PER_CELL = 8;
+__device__ __forceinline__ double fx_value(long long hi, long long lo) {
+    return (double)hi * 0x1p-24 + (double)lo * 0x1p-76;
+}
+
 int launch_move_estimate(const EstimateArgs& a, cudaStream_t s);
 int launch_move_smart(const MoveArgs& a, cudaStream_t s);
 int launch_deposit_main(const DepositArgs& a, cudaStream_t s);
@@ -154,7 +161,12 @@ struct ProfScope {
 #define LC3D_F_ALL 7
 
 struct SolveInputs {
+    // densities: ro, jx, jy, jz, or (acc != NULL) the accumulators of the
+    // deposition just before; the solve then clears those of the next one
     const double *ro, *ro_prev;           // ro_prev != NULL: ro_in = (ro + ro_prev) / 2
+    const unsigned long long* acc;
+    unsigned long long* acc_clear;
+    const double* ro_initial;
     const double *jz, *jz_prev;           // likewise for jz
     const double *jx, *jy, *jx_prev, *jy_prev, *beam;
     const double *Ex_sub, *Ey_sub, *Bx_sub, *By_sub;   // subtraction-trick terms
@@ -274,7 +286,7 @@ struct lc3d_ctx {
     double* pw[2][5];                     // predictor / corrector particles
     double* dens[4];                      // ro jx jy jz of predictor / corrector
     double* avg[6];                       // half-step averaged fields
-    unsigned long long* acc;              // deposit fixed-point accumulators, 8 planes
+    unsigned long long* acc[2];           // deposit fixed-point accumulators, 8 planes (run_step)
     size_t acc_plane;                     // plane stride in words
     unsigned* err;                        // device error flag
     unsigned* err_host;                   // pinned host word lc3d_check_error reads it into

@@ -25,8 +25,6 @@
 
 namespace {
 
-constexpr int DEP_WORDS_PER_CELL = 8;   // accumulator planes: 4 fields x (hi, lo)
-
 // ---------------------------------------------------------------------------
 // TSC weights, lcode.py:396-418. Order MP 0P PP M0 00 P0 MM 0M PM.
 // ---------------------------------------------------------------------------
@@ -232,11 +230,6 @@ __device__ __forceinline__ void fx_split(double c, long long& hi, long long& lo)
     double r = c - (t - MH);
     double t2 = r + ML;
     lo = __double_as_longlong(t2) - __double_as_longlong(ML);
-}
-
-__device__ __forceinline__ double fx_value(long long hi, long long lo) {
-    return (double)hi * 0x1p-24 +
-           (double)lo * 0x1p-76;
 }
 
 // One fine particle: coarse->fine mix (lcode.py:591-621) and the deposit

@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) oz_gemm_kernel(const __grid_c
     }
     fence_before();
     __syncthreads();
-    if (s_fail && threadIdx.x == 0) atomicOr(b.err, LC3D_FLAG_TIMEOUT);
+    if (s_fail && threadIdx.x == 0) raise_flag(b.err, LC3D_FLAG_TIMEOUT);
     if (warp == 1) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));

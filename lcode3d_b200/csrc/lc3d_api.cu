@@ -381,7 +381,6 @@ void destroy(lc3d_ctx* c) {
         if (c->avg[k]) cudaFree(c->avg[k]);
     for (int a = 0; a < 2; ++a)
         if (c->acc[a]) cudaFree(c->acc[a]);
-    if (c->err) cudaFree(c->err);
     if (c->err_host) cudaFreeHost(c->err_host);
     if (c->zeros) cudaFree(c->zeros);
     if (c->resid) cudaFree(c->resid);
@@ -612,10 +611,10 @@ int lc3d_create(const lc3d_params* p, int device, lc3d_ctx** out) {
     for (int k = 0; k < 6; ++k) LC3D_STEP(dalloc(&c->avg[k], ng));
     c->acc_plane = (ng + 31) / 32 * 32;
     for (int a = 0; a < 2; ++a) LC3D_STEP(dalloc(&c->acc[a], c->acc_plane * DEP_WORDS_PER_CELL));
-    LC3D_STEP(dalloc(&c->err, (size_t)1));
-    // pinned host word the flag is read into (a direct copy, no staging)
-    if (rc == LC3D_OK && cudaHostAlloc(&c->err_host, sizeof(unsigned), cudaHostAllocDefault) != cudaSuccess)
+    if (rc == LC3D_OK && (cudaHostAlloc(&c->err_host, LC3D_FLAGS * sizeof(unsigned), cudaHostAllocMapped) != cudaSuccess ||
+                          cudaHostGetDevicePointer(&c->err, c->err_host, 0) != cudaSuccess))
         rc = LC3D_ERR_CUDA;
+    if (rc == LC3D_OK) memset(c->err_host, 0, LC3D_FLAGS * sizeof(unsigned));
     LC3D_STEP(dalloc(&c->zeros, ng));
     LC3D_STEP(dalloc(&c->resid, (size_t)2));
     LC3D_STEP(dalloc(&c->beam_dev, ng));
@@ -1004,14 +1003,15 @@ int lc3d_set_tiles(lc3d_ctx* c, int deposit_rows, int fft_ctas_per_sm) {
 int lc3d_check_error(lc3d_ctx* c, void* stream) {
     if (!c) return LC3D_ERR_PARAM;
     DeviceGuard g(c->device);
-    LC3D_CUDA_TRY(cudaMemcpyAsync(c->err_host, c->err, sizeof(unsigned), cudaMemcpyDeviceToHost, S(stream)));
     LC3D_CUDA_TRY(cudaStreamSynchronize(S(stream)));
-    const unsigned flag = *c->err_host;
-    if (flag) LC3D_CUDA_TRY(cudaMemsetAsync(c->err, 0, sizeof(unsigned), S(stream)));
-    if (flag & LC3D_FLAG_WINDOW) return LC3D_ERR_WINDOW;
-    if (flag & LC3D_FLAG_NONFINITE) return LC3D_ERR_NONFINITE;
-    if (flag & LC3D_FLAG_TIMEOUT) return LC3D_ERR_TIMEOUT;
-    return LC3D_OK;
+    volatile unsigned* flags = c->err_host;
+    int rc = LC3D_OK;
+    if (flags[LC3D_FLAG_WINDOW]) rc = LC3D_ERR_WINDOW;
+    else if (flags[LC3D_FLAG_NONFINITE]) rc = LC3D_ERR_NONFINITE;
+    else if (flags[LC3D_FLAG_TIMEOUT]) rc = LC3D_ERR_TIMEOUT;
+    if (rc != LC3D_OK)
+        for (int k = 0; k < LC3D_FLAGS; ++k) flags[k] = 0;
+    return rc;
 }
 
 }  // extern "C"

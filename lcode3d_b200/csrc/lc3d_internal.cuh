@@ -7,10 +7,17 @@
 
 #include "../../include/lc3d.h"
 
-// Device error flag bits (the host maps them to LC3D_ERR_*).
-#define LC3D_FLAG_WINDOW 1u
-#define LC3D_FLAG_NONFINITE 2u
-#define LC3D_FLAG_TIMEOUT 4u
+// Device error flags (the host maps them to LC3D_ERR_*): words of c->err.
+#define LC3D_FLAG_WINDOW 0
+#define LC3D_FLAG_NONFINITE 1
+#define LC3D_FLAG_TIMEOUT 2
+#define LC3D_FLAGS 3
+
+// Raise a flag. The words lie in pinned host memory: the host reads them
+// after a stream synchronisation, without a copy. One store per warp.
+__device__ __forceinline__ void raise_flag(unsigned* err, int flag) {
+    if ((threadIdx.x & 31) == __ffs(__activemask()) - 1) *reinterpret_cast<volatile unsigned*>(err + flag) = 1u;
+}
 
 #define LC3D_CUDA_TRY(expr)                                                  \
     do {                                                                     \
@@ -288,8 +295,8 @@ struct lc3d_ctx {
     double* avg[6];                       // half-step averaged fields
     unsigned long long* acc[2];           // deposit fixed-point accumulators, 8 planes (run_step)
     size_t acc_plane;                     // plane stride in words
-    unsigned* err;                        // device error flag
-    unsigned* err_host;                   // pinned host word lc3d_check_error reads it into
+    unsigned* err_host;                   // error flags (LC3D_FLAGS words) in pinned host memory
+    unsigned* err;                        // ... and their device address
     double* zeros;                        // N x N zeros (absent beam)
     unsigned long long* resid;            // predicted-step residual maxima (2 words, double bits)
     double* diag_w;                       // zn diagnostic: Gaussian weights, then partial sums

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(LC3D_MOVE_THREADS, 1) move_smart_kernel(MoveAr
     Tsc t = tsc_weights(x_half, y_half, a.N, a.h, a.inv_h);
     if (!tsc_in_grid(t, a.N)) {
         // the reference would read out of bounds here; flag and keep prev
-        atomicOr(a.err, LC3D_FLAG_WINDOW);
+        raise_flag(a.err, LC3D_FLAG_WINDOW);
         a.out_x[k] = x_offt;
         a.out_y[k] = y_offt;
         a.out_px[k] = opx;
@@ -487,7 +487,7 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
 #pragma unroll
     for (int u = 0; u < DEP_RPW; ++u) {
         const bool idx = pi[u] >= 0 && pi[u] < a.Nc && ni[u] >= 0 && ni[u] < a.Nc;
-        if (row_ok[u] && col_ok && !(idx && col_idx)) atomicOr(a.err, LC3D_FLAG_WINDOW);
+        if (row_ok[u] && col_ok && !(idx && col_idx)) raise_flag(a.err, LC3D_FLAG_WINDOW);
         if (!idx) pi[u] = ni[u] = 0;   // nobody uses that row of the table
         ok[u] = row_ok[u] && col_ok && idx && col_idx;
     }
@@ -557,7 +557,8 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
             // also false for NaN
             const bool fin = fabs(f[u].dro) < FX_MAX && fabs(f[u].djx) < FX_MAX && fabs(f[u].djy) < FX_MAX &&
                              fabs(f[u].djz) < FX_MAX;
-            if (ok[u] && !(in && fin)) atomicOr(a.err, in ? LC3D_FLAG_NONFINITE : LC3D_FLAG_WINDOW);
+            if (ok[u] && !in) raise_flag(a.err, LC3D_FLAG_WINDOW);
+            if (ok[u] && in && !fin) raise_flag(a.err, LC3D_FLAG_NONFINITE);
             cell[u] = ok[u] && in && fin ? (i << 16) | j : -1;
             if (cell[u] >= 0) {
                 const int k = (row0 + u) * DEP_TW + lane;

@@ -148,7 +148,13 @@ def _key(p, device):
     return tuple(getattr(p, f) for f, _ in p._fields_) + (device,)
 
 
+# the handle of the current stream without a Stream object, where torch has it
+_raw_stream = getattr(torch._C, '_cuda_getCurrentRawStream', None)
+
+
 def _stream():
+    if _raw_stream is not None:
+        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
@@ -272,6 +278,9 @@ def _empty(shape):
 
 
 def _f64(a, shape=None):
+    if (isinstance(a, torch.Tensor) and a.is_cuda and a.dtype == torch.float64 and a.is_contiguous() and
+            a.device == _device() and (shape is None or tuple(a.shape) == tuple(shape))):
+        return a   # already what the C call takes: no conversion calls
     t = to_device(a, torch.float64)
     if shape is not None and tuple(t.shape) != tuple(shape):
         t = t.expand(shape).contiguous()
@@ -416,7 +425,7 @@ def calculate_Bz(config, jx, jy):
 def move_estimate_wo_fields(config, m, x_init, y_init, prev_x_offt, prev_y_offt, px, py, pz):
     """Field-free drift with coordinate reflection (lcode.py:369-391)."""
     s = solver_for(config)
-    shape = tuple(to_device(prev_x_offt).shape)
+    shape = tuple(_f64(prev_x_offt).shape)
     a = [_f64(v, shape) for v in (m, x_init, y_init, prev_x_offt, prev_y_offt, px, py, pz)]
     ox, oy = _empty(shape), _empty(shape)
     check(lib.lc3d_move_estimate_wo_fields(s.ctx, *[_ptr(v) for v in a], _ptr(ox), _ptr(oy),
@@ -429,7 +438,7 @@ def move_smart(config, m, q, x_init, y_init, x_prev_offt, y_prev_offt,
                Ex_avg, Ey_avg, Ez_avg, Bx_avg, By_avg, Bz_avg):
     """Pusher with half-step TSC field interpolation (lcode.py:704-823)."""
     s = solver_for(config)
-    shape = tuple(to_device(x_prev_offt).shape)
+    shape = tuple(_f64(x_prev_offt).shape)
     part = [_f64(v, shape) for v in (m, q, x_init, y_init, x_prev_offt, y_prev_offt,
                                      estimated_x_offt, estimated_y_offt, px_prev, py_prev, pz_prev)]
     g = _grid(config)
@@ -446,7 +455,7 @@ def deposit(config, ro_initial, x_offt, y_offt, m, q, px, py, pz, virt_params):
     jx, jy, jz, plus ro_initial (lcode.py:666-689)."""
     s = solver_for(config)
     s.set_virt(virt_params)
-    shape = tuple(to_device(x_offt).shape)
+    shape = tuple(_f64(x_offt).shape)
     part = [_f64(v, shape) for v in (x_offt, y_offt, m, q, px, py, pz)]
     g = _grid(config)
     roi = None

@@ -41,7 +41,7 @@
 
 namespace {
 
-constexpr int F64_THREADS = 256;
+constexpr int F64_THREADS = 512;          // at most
 constexpr int MAX_MIDS = 6;
 
 struct F64Plan {
@@ -322,11 +322,13 @@ __device__ __forceinline__ void first_pass(const Shared<LF>& S, const F64Plan& p
 }
 
 // Last pass on the way back: store(f, j, v), v[reg_of(s)] the transform at
-// j + s M1 (s < R1/2) or at the mirror (R1 - s) M1 - j (the others).
+// j + s M1 (s < R1/2) or at the mirror (R1 - s) M1 - j (the others);
+// ahead(f, j) comes before the task's shared-memory reads.
 // ROWS_FAST: lanes along the columns (rows are written), else along the pairs
 // (a transposed line is written).
-template <int R1, bool ROWS_FAST, int LF, typename Store>
-__device__ __forceinline__ void last_pass(const Shared<LF>& S, const F64Plan& p, const double2* tw, int type, const Store& store) {
+template <int R1, bool ROWS_FAST, int LF, typename Ahead, typename Store>
+__device__ __forceinline__ void last_pass(const Shared<LF>& S, const F64Plan& p, const double2* tw, int type, const Ahead& ahead,
+                                          const Store& store) {
     const float inv_ncol = 1.0f / (float)p.ncol, inv_rl = 1.0f / (float)p.RL;
     const int per = p.M1 / p.RL, step = per * S.PITCH;
     const unsigned neg = type ? 0x80000000u : 0u;
@@ -346,6 +348,7 @@ __device__ __forceinline__ void last_pass(const Shared<LF>& S, const F64Plan& p,
         const int b1 = div_small(j2, inv_rl), q1 = j2 - b1 * p.RL;
         const double2 *s0 = S.at(q0 * p.PB + b0, f), *s1 = S.at(q1 * p.PB + b1, f);
         const double2 w = __ldg(tw + j);
+        ahead(f, j);
         double2 v[R1];
         v[0] = s0[0];
         powers<R1 / 2>(w, [&](int m, double2 wm) {
@@ -486,7 +489,7 @@ __device__ __forceinline__ void load_rows(const Shared<LF>& S, const F64Plan& p,
 
 // A: rows along axis 1, out[p][grid row].
 template <int LF>
-__global__ void __launch_bounds__(F64_THREADS, 2) fft64_a_kernel(const __grid_constant__ F64Batch b) {
+__global__ void __launch_bounds__(F64_THREADS) fft64_a_kernel(const __grid_constant__ F64Batch b) {
     extern __shared__ __align__(16) unsigned char fft64_smem[];
     const F64Plan& p = b.p;
     const Shared<LF> S{reinterpret_cast<double2*>(fft64_smem)};
@@ -525,7 +528,7 @@ __global__ void __launch_bounds__(F64_THREADS, 2) fft64_a_kernel(const __grid_co
 
 // B: rows along axis 0: forth, times Lambda, back; out[grid row][p].
 template <int LF>
-__global__ void __launch_bounds__(F64_THREADS, 2) fft64_b_kernel(const __grid_constant__ F64Batch b) {
+__global__ void __launch_bounds__(F64_THREADS) fft64_b_kernel(const __grid_constant__ F64Batch b) {
     extern __shared__ __align__(16) unsigned char fft64_smem[];
     __shared__ double red[F64_THREADS / 32];
     const F64Plan& p = b.p;
@@ -572,7 +575,7 @@ __global__ void __launch_bounds__(F64_THREADS, 2) fft64_b_kernel(const __grid_co
     double psum = 0.0;
     auto store = [&](auto RC) {
         constexpr int R1 = decltype(RC)::value;
-        last_pass<R1, false>(S, p, b.tw, F.type, [&](int f, int j, double2 (&v)[R1]) {
+        last_pass<R1, false>(S, p, b.tw, F.type, [](int, int) {}, [&](int f, int j, double2 (&v)[R1]) {
             // a mirror written twice (columns 0 and M1 / 2) is written by one
             // thread, so which value stays does not vary
             double* o = F.out + row0 + 2 * f;
@@ -620,7 +623,7 @@ __device__ __forceinline__ int d_row(int r, int N, int border) {
 
 // D: rows along axis 1, back only; the field itself, finalised.
 template <int LF>
-__global__ void __launch_bounds__(F64_THREADS, 2) fft64_d_kernel(const __grid_constant__ F64Batch b) {
+__global__ void __launch_bounds__(F64_THREADS) fft64_d_kernel(const __grid_constant__ F64Batch b) {
     extern __shared__ __align__(16) unsigned char fft64_smem[];
     __shared__ double s_mean;
     const F64Plan& p = b.p;
@@ -681,37 +684,45 @@ __global__ void __launch_bounds__(F64_THREADS, 2) fft64_d_kernel(const __grid_co
     const double mean = F.partial ? s_mean : 0.0;
     auto store = [&](auto RC) {
         constexpr int R1 = decltype(RC)::value;
-        last_pass<R1, true>(S, p, b.tw, F.type, [&](int f, int j, double2 (&v)[R1]) {
-            const int r = row0 + 2 * f;
-            const int ga = d_row(r, p.N, F.border), gb = d_row(r + 1, p.N, F.border);
+        // the previous field of the pair's first row is loaded before the
+        // pass's shared-memory reads and butterfly, that of the second row as
+        // the first one's values are stored
+        double old[R1];
+        auto row_of = [&](int f, int h) { return d_row(row0 + 2 * f + h, p.N, F.border); };
+        auto n_of = [&](int j, int s) { return s < R1 / 2 ? j + s * p.M1 : (R1 - s) * p.M1 - j; };
+        auto ahead = [&](int f, int j) {
+            const int g = row_of(f, 0);
+            if (F.avg && g >= 0) {
+                const double* pr = F.prev + g * p.N;
+#pragma unroll
+                for (int s = 0; s < R1; ++s) old[s] = pr[n_of(j, s)];
+            }
+        };
+        last_pass<R1, true>(S, p, b.tw, F.type, ahead, [&](int f, int j, double2 (&v)[R1]) {
             const unsigned neg = F.type ? 0x80000000u : 0u;
             const bool interior = j > 0 && 2 * j != p.M1;   // the other columns are their own mirrors
             if (F.type && j == 0) v[reg_of<R1>(0)] = v[reg_of<R1>(R1 / 2)] = mk(0.0, 0.0);
-            // half of a row of the pair at a time, its loads before its stores
+            const int gb = row_of(f, 1);
+            const double* next = F.avg && gb >= 0 ? F.prev + gb * p.N : nullptr;
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                const int g = h & 1 ? gb : ga, s0 = h & 2 ? R1 / 2 : 0;
+            for (int h = 0; h < 2; ++h) {
+                const int g = h ? gb : row_of(f, 0);
                 if (g < 0) continue;
-                const int at = g * p.N;
-                double* o = F.out ? F.out + at : nullptr;
-                double* a = F.avg ? F.avg + at : nullptr;
-                const double* pr = F.prev + at;
-                double old[R1 / 2];
-                if (a)
+                double* o = F.out ? F.out + g * p.N : nullptr;
+                double* a = F.avg ? F.avg + g * p.N : nullptr;
 #pragma unroll
-                    for (int u = 0; u < R1 / 2; ++u)
-                        old[u] = pr[s0 ? (R1 / 2 - u) * p.M1 - j : j + u * p.M1];
-#pragma unroll
-                for (int u = 0; u < R1 / 2; ++u) {
-                    if (s0 && !interior && !(u == 0 && j == 0)) continue;
-                    const int n = s0 ? (R1 / 2 - u) * p.M1 - j : j + u * p.M1;
-                    const double2 z = v[reg_of<R1>(s0 + u)];
-                    double x = h & 1 ? z.y : z.x;
-                    if (s0) x = flip(x, neg);
+                for (int s = 0; s < R1; ++s) {
+                    const int n = n_of(j, s);
+                    const double2 z = v[reg_of<R1>(s)];
+                    double x = h ? z.y : z.x;
+                    if (s >= R1 / 2) x = flip(x, neg);
                     x -= mean;
-                    if (F.variant_a) x = 2 * x - old[u];
-                    if (o) o[n] = x;
-                    if (a) a[n] = (x + old[u]) / 2;
+                    if (F.variant_a) x = 2 * x - old[s];
+                    if (s < R1 / 2 || interior || (s == R1 / 2 && j == 0)) {
+                        if (o) o[n] = x;
+                        if (a) a[n] = (x + old[s]) / 2;
+                    }
+                    if (h == 0 && next) old[s] = next[n];
                 }
             }
         });
@@ -736,7 +747,7 @@ __global__ void lam_order_kernel(const double* __restrict__ lam, int ld, const i
     out[(size_t)t * ld_out + (swap ? c ^ 1 : c)] = swap ? -v : v;
 }
 
-constexpr int F64_SMALL = 400;   // rows: see fft64_init
+constexpr int F64_SMALL = 400, F64_MEDIUM = 1100;   // rows: see fft64_init
 
 // The radices of P. One middle radix where there is such a plan: two passes
 // need radices so large, and four so many barriers, that both are slower (us
@@ -831,15 +842,22 @@ int fft64_init(lc3d_ctx* c) {
     const int N = c->N, L = p.L;
     F64State* s = new F64State();
     c->fft64 = s;
-    // Pairs and threads per CTA. Eight pairs store whole lines and fill two
-    // CTAs of an SM from about 400 rows on; smaller grids take four pairs on
-    // as many threads, for twice the CTAs (us per xi step, F = 8 / F = 4: 161^2
-    // 79.3 / 76.1, 321^2 129.0 / 119.4, 481^2 239.4 / 240.5, 641^2 363.7 /
-    // 429.5, 1025^2 963.5 / 971.2; F = 4 on 128 threads above 400 rows).
-    const bool small = N < F64_SMALL;
-    p.lf = small ? 2 : 3;
+    // Pairs and threads per CTA: 256 threads and two CTAs per SM where the
+    // shared memory allows, else 512 threads and one. Eight pairs store whole
+    // lines and fill the SMs from about 400 rows on; smaller grids take four,
+    // for twice the CTAs, and so do those of 700 to 1100 rows, of which eight
+    // pairs fit an SM once and four twice (us per xi step, F = 8 / F = 4: 161^2
+    // 79.3 / 76.1, 321^2 129.0 / 119.4, 401^2 199 / 222, 641^2 372 / 430; 801^2
+    // 621 / 600, 961^2 800 / 778, 1025^2 927 / 913, 1153^2 1118 / 1156, 1281^2
+    // 1482 / 1549).
+    auto twice = [&](int lf) {
+        p.lf = lf;
+        return 2 * (smem_bytes(p) + 2048) <= 228 * 1024;
+    };
+    int lf = 3;
+    if (N < F64_SMALL || (N <= F64_MEDIUM && !twice(3) && twice(2))) lf = 2;
+    s->threads = twice(lf) ? 256 : 512;
     if (smem_bytes(p) > F64_MAX_SMEM) p.lf = 2;
-    s->threads = small || p.lf == 3 ? F64_THREADS : F64_THREADS / 2;
     if (smem_bytes(p) > F64_MAX_SMEM) return LC3D_ERR_SIZE;
     s->p = p;
     s->pitch = fft64_pitch(N);

@@ -853,16 +853,17 @@ struct lc3d_predictor {
     float *y = nullptr, *target = nullptr;
     // gradients (float32 NHWC)
     float *g_d1 = nullptr, *g_d2 = nullptr, *g_e3 = nullptr, *g_p2 = nullptr, *g_p1 = nullptr;
-    // tensor-core backward data pass: the bf16 output gradient of the layer
-    // in hand, the flipped transposed bf16 weights of every layer, zeros for
+    // tensor-core backward passes: the bf16 output gradients of two layers, the flipped transposed bf16 weights of every layer, zeros for
     // the bias, and the convolution arguments of each layer's pass
-    __nv_bfloat16* g_bf = nullptr;
+    __nv_bfloat16* g_bf[2] = {nullptr, nullptr};   // layer l uses g_bf[l & 1]
     __nv_bfloat16* wt = nullptr;
     long long wt_off[NLAYERS];
     float* zero_bias = nullptr;
     ConvArgs bconv[NLAYERS];
     WgradArgs wg[NLAYERS];         // tensor-core weight gradient of each layer
     dim3 wg_grid[NLAYERS];
+    cudaStream_t wg_stream = nullptr;              // the weight-gradient passes' stream
+    cudaEvent_t ev_grad[NLAYERS] = {}, ev_wg[NLAYERS] = {};   // layer l's g_bf written; read by its weight pass
     unsigned* err = nullptr;
     double* scale = nullptr;       // [23] per-sample channel scales (device)
     double* partial = nullptr;     // [STAT_BLOCKS][18]
@@ -917,7 +918,7 @@ int setup_bconv(lc3d_predictor* P, int l) {
     const int CGp = grad_channels(l);
     ConvArgs& a = P->bconv[l];
     memset(&a, 0, sizeof(a));
-    LC3D_TRY(make_map_2d(&a.tin, P->g_bf, L.NP, CGp, TILE_PIX));
+    LC3D_TRY(make_map_2d(&a.tin, P->g_bf[l & 1], L.NP, CGp, TILE_PIX));
     LC3D_TRY(make_map_2d(&a.twt, P->wt + P->wt_off[l], 9LL * d.cin, CGp, d.cin));
     a.bias = P->zero_bias;
     a.out_f32 = 1;
@@ -934,7 +935,7 @@ int setup_wgrad(lc3d_predictor* P, int l, const __nv_bfloat16* x) {
     const Level& L = P->lv[d.level];
     WgradArgs& a = P->wg[l];
     memset(&a, 0, sizeof(a));
-    LC3D_TRY(make_map_2d(&a.tg, P->g_bf, L.NP, grad_channels(l), WG_PIX));
+    LC3D_TRY(make_map_2d(&a.tg, P->g_bf[l & 1], L.NP, grad_channels(l), WG_PIX));
     LC3D_TRY(make_map_2d(&a.tx, x, L.NP, d.cin, WG_PIX));
     a.dw = P->grad + P->w_off[l];
     a.Cout = d.cout;
@@ -952,7 +953,7 @@ int setup_wgrad(lc3d_predictor* P, int l, const __nv_bfloat16* x) {
     return LC3D_OK;
 }
 
-// dW of layer l from its output gradient in P->g_bf.
+// dW of layer l from its output gradient in g_bf.
 int bwd_weights_tc(lc3d_predictor* P, int l, cudaStream_t s) {
     const WgradArgs& a = P->wg[l];
     conv_wgrad_tc_kernel<<<P->wg_grid[l], CONV_THREADS, wgrad_smem_bytes(), s>>>(a);
@@ -960,7 +961,7 @@ int bwd_weights_tc(lc3d_predictor* P, int l, cudaStream_t s) {
     return LC3D_OK;
 }
 
-// dx = dL/d(input of layer l) from P->g_bf, zeroed where mask <= 0.
+// dx = dL/d(input of layer l) from g_bf, zeroed where mask <= 0.
 int bwd_data_tc(lc3d_predictor* P, int l, const __nv_bfloat16* mask, float* dx, cudaStream_t s) {
     ConvArgs a = P->bconv[l];
     a.out = dx;
@@ -996,35 +997,56 @@ int backward(lc3d_predictor* P, float* loss, cudaStream_t s) {
                                                                 grad_channels(l), P->wt + P->wt_off[l]);
     }
     LC3D_CUDA_TRY(cudaGetLastError());
-    // each layer: its output gradient in bf16 (P->g_bf) with the bias
-    // gradient, then the weight and data passes on it
+    // Each layer: its output gradient in bf16 (g_bf[l & 1]) with the bias
+    // gradient, then the data pass on this stream and the weight pass on a
+    // second one: the weight pass waits on its MMAs with one CTA per SM, the
+    // data pass on its loads with five (641^2: 866 -> 784 us a training
+    // sample). A layer's gradient is written over the one of two layers before
+    // once that layer's weight pass has read it.
     auto db = [&](int l) { return P->grad + P->b_off[l]; };
     auto grid = [&](const Level& L, int C) {   // CTAs of a gradient kernel: a few pixels per thread, six CTAs per SM at most
         return std::min(blocks_for((long long)L.NP * (C / 8), GRAD_THREADS * 4), 148u * 6);
     };
+    auto before = [&](int l) -> int {   // g_bf[l & 1] is free
+        if (l + 2 < NLAYERS) LC3D_CUDA_TRY(cudaStreamWaitEvent(s, P->ev_wg[l + 2], 0));
+        return LC3D_OK;
+    };
+    auto weights = [&](int l) -> int {
+        LC3D_CUDA_TRY(cudaEventRecord(P->ev_grad[l], s));
+        LC3D_CUDA_TRY(cudaStreamWaitEvent(P->wg_stream, P->ev_grad[l], 0));
+        LC3D_TRY(bwd_weights_tc(P, l, P->wg_stream));
+        LC3D_CUDA_TRY(cudaEventRecord(P->ev_wg[l], P->wg_stream));
+        return LC3D_OK;
+    };
     // conv6: d1 -> y
-    loss_kernel<<<grid(l0, 8), GRAD_THREADS, 0, s>>>(P->y, P->target, P->g_bf, l0, loss, db(5));
-    LC3D_TRY(bwd_weights_tc(P, 5, s));
+    loss_kernel<<<grid(l0, 8), GRAD_THREADS, 0, s>>>(P->y, P->target, P->g_bf[1], l0, loss, db(5));
+    LC3D_TRY(weights(5));
     LC3D_TRY(bwd_data_tc(P, 5, P->d1, P->g_d1, s));
     // conv5: d2 -> u2
-    downsum_kernel<<<grid(l1, 32), GRAD_THREADS, 0, s>>>(P->g_d1, l0, P->g_bf, l1, 32, db(4));
-    LC3D_TRY(bwd_weights_tc(P, 4, s));
+    downsum_kernel<<<grid(l1, 32), GRAD_THREADS, 0, s>>>(P->g_d1, l0, P->g_bf[0], l1, 32, db(4));
+    LC3D_TRY(weights(4));
     LC3D_TRY(bwd_data_tc(P, 4, P->d2, P->g_d2, s));
     // conv4: e3 -> u3
-    downsum_kernel<<<grid(l2, 64), GRAD_THREADS, 0, s>>>(P->g_d2, l1, P->g_bf, l2, 64, db(3));
-    LC3D_TRY(bwd_weights_tc(P, 3, s));
+    LC3D_TRY(before(3));
+    downsum_kernel<<<grid(l2, 64), GRAD_THREADS, 0, s>>>(P->g_d2, l1, P->g_bf[1], l2, 64, db(3));
+    LC3D_TRY(weights(3));
     LC3D_TRY(bwd_data_tc(P, 3, P->e3, P->g_e3, s));
     // conv3: p2 -> e3
-    grad_bf16_kernel<<<grid(l2, 128), GRAD_THREADS, 0, s>>>(P->g_e3, P->g_bf, l2, 128, db(2));
-    LC3D_TRY(bwd_weights_tc(P, 2, s));
+    LC3D_TRY(before(2));
+    grad_bf16_kernel<<<grid(l2, 128), GRAD_THREADS, 0, s>>>(P->g_e3, P->g_bf[0], l2, 128, db(2));
+    LC3D_TRY(weights(2));
     LC3D_TRY(bwd_data_tc(P, 2, nullptr, P->g_p2, s));
     // conv2: p1 -> e2
-    pool_bwd_mask_kernel<<<grid(l1, 64), GRAD_THREADS, 0, s>>>(P->g_d2, P->e2, l1, P->g_p2, l2, 64, P->g_bf, db(1));
-    LC3D_TRY(bwd_weights_tc(P, 1, s));
+    LC3D_TRY(before(1));
+    pool_bwd_mask_kernel<<<grid(l1, 64), GRAD_THREADS, 0, s>>>(P->g_d2, P->e2, l1, P->g_p2, l2, 64, P->g_bf[1], db(1));
+    LC3D_TRY(weights(1));
     LC3D_TRY(bwd_data_tc(P, 1, nullptr, P->g_p1, s));
     // conv1: x0 -> e1
-    pool_bwd_mask_kernel<<<grid(l0, 32), GRAD_THREADS, 0, s>>>(P->g_d1, P->e1, l0, P->g_p1, l1, 32, P->g_bf, db(0));
-    LC3D_TRY(bwd_weights_tc(P, 0, s));
+    LC3D_TRY(before(0));
+    pool_bwd_mask_kernel<<<grid(l0, 32), GRAD_THREADS, 0, s>>>(P->g_d1, P->e1, l0, P->g_p1, l1, 32, P->g_bf[0], db(0));
+    LC3D_TRY(weights(0));
+    // the second stream is in order: its last pass ends the backward pass
+    LC3D_CUDA_TRY(cudaStreamWaitEvent(s, P->ev_wg[0], 0));
     LC3D_CUDA_TRY(cudaGetLastError());
     return LC3D_OK;
 }
@@ -1079,7 +1101,7 @@ int lc3d_predictor_create(int grid_steps, int device, lc3d_predictor** out) {
             if (l == 0) continue;
             wtot += 9LL * LAYERS[l].cin * grad_channels(l);
         }
-        PA(P->g_bf, gmax); PA(P->wt, (size_t)wtot); PA(P->zero_bias, 128);
+        PA(P->g_bf[0], gmax); PA(P->g_bf[1], gmax); PA(P->wt, (size_t)wtot); PA(P->zero_bias, 128);
     }
 #undef PA
     if (rc == LC3D_OK) rc = setup_conv(P, 0, P->x0, P->e1);
@@ -1088,6 +1110,11 @@ int lc3d_predictor_create(int grid_steps, int device, lc3d_predictor** out) {
     if (rc == LC3D_OK) rc = setup_conv(P, 3, P->e3, P->u3);
     if (rc == LC3D_OK) rc = setup_conv(P, 4, P->d2, P->u2);
     if (rc == LC3D_OK) rc = setup_conv(P, 5, P->d1, P->y);
+    if (rc == LC3D_OK && cudaStreamCreateWithFlags(&P->wg_stream, cudaStreamNonBlocking) != cudaSuccess) rc = LC3D_ERR_CUDA;
+    for (int l = 0; l < NLAYERS && rc == LC3D_OK; ++l)
+        if (cudaEventCreateWithFlags(&P->ev_grad[l], cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&P->ev_wg[l], cudaEventDisableTiming) != cudaSuccess)
+            rc = LC3D_ERR_CUDA;
     for (int l = 1; l < NLAYERS && rc == LC3D_OK; ++l) rc = setup_bconv(P, l);
     {   // the input activation of each layer, for its weight gradient
         const __nv_bfloat16* xin[NLAYERS] = {P->x0, P->p1, P->p2, P->e3, P->d2, P->d1};
@@ -1116,6 +1143,11 @@ int lc3d_predictor_destroy(lc3d_predictor* P) {
     if (!P) return LC3D_OK;
     PredDevice g(P->device);
     for (void* q : P->allocs) cudaFree(q);
+    for (int l = 0; l < NLAYERS; ++l) {
+        if (P->ev_grad[l]) cudaEventDestroy(P->ev_grad[l]);
+        if (P->ev_wg[l]) cudaEventDestroy(P->ev_wg[l]);
+    }
+    if (P->wg_stream) cudaStreamDestroy(P->wg_stream);
     delete P;
     return LC3D_OK;
 }

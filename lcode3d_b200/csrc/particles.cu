@@ -401,6 +401,12 @@ constexpr int DEP_WIN = 352;                // window cells, (rows + 2) (columns
 // 132 / 160 / 137 / 138, 161^2 86.5 / 86.1 / 83.2 / 84.3).
 __host__ __device__ constexpr int dep_threads(int ti) { return (ti + DEP_RPW - 1) / DEP_RPW * 32; }
 
+// Staged particle of column `col` of a row: even columns, then odd ones, at a
+// pitch of 36. Lanes of neighbouring cells read every other column, lanes of a
+// warp write all of them; both touch distinct banks.
+constexpr int DEP_ROW = 36;
+__device__ __forceinline__ int dep_slot(int col) { return (col >> 1) + (col & 1) * 20; }
+
 template <int TI>
 __host__ __device__ constexpr size_t dep_table_words() {   // double2 words: the row tables, then the window
     constexpr size_t table = (size_t)TI * DEP_CMAX * 4, win = 2 * DEP_WIN;
@@ -408,7 +414,7 @@ __host__ __device__ constexpr size_t dep_table_words() {   // double2 words: the
 }
 template <int TI>
 constexpr size_t dep_smem() {
-    return ((size_t)TI * DEP_TW * 3 + dep_table_words<TI>()) * sizeof(double2)   // (xl, yl), (ro, jx), (jy, jz); table
+    return ((size_t)TI * DEP_ROW * 3 + dep_table_words<TI>()) * sizeof(double2)   // (xl, yl), (ro, jx), (jy, jz); table
            + (TI + 1) * DEP_CELLS * sizeof(unsigned);                            // masks, rows in use
 }
 
@@ -426,14 +432,14 @@ __device__ __forceinline__ double2 coarse_pair(const DepositArgs& a, int k, int 
 
 template <int TI>
 __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, int tile_y) {
-    constexpr int T = dep_threads(TI), P = TI * DEP_TW;
+    constexpr int T = dep_threads(TI), P = TI * DEP_ROW;
     static_assert(TI <= 32, "masks of 32 bits");
     extern __shared__ __align__(16) double smem_f64[];
     double2* s_pos = reinterpret_cast<double2*>(smem_f64);               // [P] cell offsets
     double2* s_v01 = s_pos + P;                                          // [P] ro, jx
     double2* s_v23 = s_v01 + P;                                          // [P] jy, jz
     double2* s_R = s_v23 + P;                                            // [TI][DEP_CMAX][4]; then the window
-    double* s_win = reinterpret_cast<double*>(s_R);                      // [4][DEP_WIN]
+    double2* s_win = s_R;                                                // [2][DEP_WIN]: ro, jx; jy, jz
     unsigned* s_mask = reinterpret_cast<unsigned*>(s_R + dep_table_words<TI>());   // [TI][DEP_CELLS]
     unsigned* s_rows = s_mask + TI * DEP_CELLS;                          // [DEP_CELLS]
     __shared__ int s_bb[4];                                              // imin imax jmin jmax
@@ -561,7 +567,7 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
             if (ok[u] && in && !fin) raise_flag(a.err, LC3D_FLAG_NONFINITE);
             cell[u] = ok[u] && in && fin ? (i << 16) | j : -1;
             if (cell[u] >= 0) {
-                const int k = (row0 + u) * DEP_TW + lane;
+                const int k = (row0 + u) * DEP_ROW + dep_slot(lane);
                 s_pos[k] = make_double2(xl, yl);
                 s_v01[k] = make_double2(f[u].dro, f[u].djx);
                 s_v23[k] = make_double2(f[u].djy, f[u].djz);
@@ -591,16 +597,18 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
     __syncthreads();   // the bounding box; the row tables are done with
     if (s_bb[0] > s_bb[1]) return;   // no particle (uniform)
     const int oj = s_bb[2], mj = min(s_bb[3] - oj + 1, DEP_SIDE);   // the first column of cells with particles, columns
-    const int strip_rows = min(DEP_SIDE, DEP_CELLS / mj), wj = mj + 2;
-    const int strips = min((s_bb[1] - s_bb[0]) / strip_rows + 1, DEP_STRIPS);
+    // quotients of small integers: (a + 0.5) / b lies at least 0.5 / b from an
+    // integer, more than the float rounding
+    const float inv_mj = 1.0f / (float)mj;
+    const int strip_rows = min(DEP_SIDE, __float2int_rz((DEP_CELLS + 0.5f) * inv_mj)), wj = mj + 2;
+    const int strips = min(__float2int_rz(((float)(s_bb[1] - s_bb[0]) + 0.5f) / (float)strip_rows) + 1, DEP_STRIPS);
     for (int strip = 0; strip < strips; ++strip) {
         // this window's cells with particles: mi rows from oi, mj columns from
         // oj; the window holds one cell more on each side
         const int oi = s_bb[0] + strip * strip_rows, mi = min(s_bb[1] - oi + 1, strip_rows);
         const int nwin = (mi + 2) * wj, ncell = mi * mj;
         for (int w = t; w < nwin; w += T)
-#pragma unroll
-            for (int f = 0; f < 4; ++f) s_win[f * DEP_WIN + w] = 0.0;
+            s_win[w] = s_win[DEP_WIN + w] = make_double2(0.0, 0.0);
         if (strip) {   // the first window's masks were cleared above
             uint4* z = reinterpret_cast<uint4*>(s_mask);
             for (int w = t; w < (TI + 1) * DEP_CELLS / 4; w += T) z[w] = make_uint4(0u, 0u, 0u, 0u);
@@ -615,7 +623,7 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
                 atomicOr(&s_mask[row * DEP_CELLS + c], 1u << lane);
                 atomicOr(&s_rows[c], 1u << row);
             } else if (strip == 0 && (j >= mj || i >= strips * strip_rows)) {   // in no window
-                const int k = row * DEP_TW + lane;
+                const int k = row * DEP_ROW + dep_slot(lane);
                 unsigned long long* g = a.acc + (size_t)(oi + i - 1) * N + (oj + j - 1);
                 double wx[3], wy[3];
                 tsc_axis(s_pos[k].x, wx[0], wx[1], wx[2]);
@@ -632,7 +640,6 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
         __syncthreads();   // masks complete, window cleared
 
         // ---- phase 2: one cell per thread ----
-        const float inv_mj = 1.0f / (float)mj;
         for (int r0 = 0; r0 < ncell; r0 += T) {
             const int c = r0 + t;
             unsigned rows = c < ncell ? s_rows[c] : 0u, m = 0;
@@ -649,9 +656,9 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
                     const int r = __ffs(rows) - 1;
                     rows &= rows - 1;
                     m = mk[r * DEP_CELLS];
-                    base = r * DEP_TW;
+                    base = r * DEP_ROW;
                 }
-                const int k = base + __ffs(m) - 1;
+                const int k = base + dep_slot(__ffs(m) - 1);
                 m &= m - 1;
                 const double2 pos = s_pos[k], v01 = s_v01[k], v23 = s_v23[k];
                 double wx[3], wy[3];
@@ -667,15 +674,15 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
                         for (int dj = 0; dj < 3; ++dj) acc[f][di * 3 + dj] = fma(vx, wy[dj], acc[f][di * 3 + dj]);
                     }
             }
-            // (c + 0.5) / mj lies at least 0.5 / mj from an integer, more than the float rounding
             const int ci = __float2int_rz(((float)c + 0.5f) * inv_mj), cj = c - ci * mj;
-            double* w = s_win + ci * wj + cj;
+            double2* w = s_win + ci * wj + cj;
 #pragma unroll
             for (int e = 0; e < 9; ++e) {
                 if (any) {
-                    double* we = w + (e / 3) * wj + e % 3;
-#pragma unroll
-                    for (int f = 0; f < 4; ++f) we[f * DEP_WIN] += acc[f][e];
+                    double2* we = w + (e / 3) * wj + e % 3;
+                    const double2 x = we[0], y = we[DEP_WIN];
+                    we[0] = make_double2(x.x + acc[0][e], x.y + acc[1][e]);
+                    we[DEP_WIN] = make_double2(y.x + acc[2][e], y.y + acc[3][e]);
                 }
                 __syncthreads();
             }
@@ -686,11 +693,11 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
         for (int w = t; w < nwin; w += T) {
             const int ci = __float2int_rz(((float)w + 0.5f) * inv_wj), cj = w - ci * wj;
             unsigned long long* g = a.acc + (size_t)(oi - 1 + ci) * N + (oj - 1 + cj);
+            const double2 x = s_win[w], y = s_win[DEP_WIN + w];
+            const double v[4] = {x.x, x.y, y.x, y.y};
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                const double v = s_win[f * DEP_WIN + w];
-                if (v != 0.0) fx_add(g + 2 * f * NN, g + (2 * f + 1) * NN, 0, v);
-            }
+            for (int f = 0; f < 4; ++f)
+                if (v[f] != 0.0) fx_add(g + 2 * f * NN, g + (2 * f + 1) * NN, 0, v[f]);
         }
         if (strip + 1 < strips) __syncthreads();   // the window is read; the next one clears it
     }

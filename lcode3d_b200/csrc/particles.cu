@@ -41,6 +41,38 @@ __device__ __forceinline__ double div_h(double x, double h, double inv_h) {
     return fma(fma(-q0, h, x), inv_h, q0);
 }
 
+// sqrt(S) and 1 / sqrt(S) without branches (the library's functions end each
+// block of instructions with a test for their slow path, so chains of several
+// particles, or of one particle's quotients, do not overlap): Goldschmidt's
+// iteration for sqrt(S) and 1 / (2 sqrt(S)) from the hardware's approximation,
+// both corrected by their exact residuals (Markstein). S normal and well
+// inside the range: in_fast_range.
+__device__ __forceinline__ void sqrt_fast(double S, double& g, double& inv) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(S));
+    double h = .5 * y;
+    g = S * y;
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+        const double e = fma(-g, h, .5);
+        g = fma(g, e, g);
+        h = fma(h, e, h);
+    }
+    g = fma(fma(-g, g, S), h, g);
+    inv = h + h;
+    inv = fma(inv, fma(-g, inv, 1.0), inv);
+}
+__device__ __forceinline__ bool in_fast_range(double S) { return S > 0x1p-900 && S < 0x1p900; }
+
+// 1 / d by Newton's iteration, for a quotient x / d = div_h(x, d, recip_fast(d)).
+__device__ __forceinline__ double recip_fast(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+#pragma unroll
+    for (int it = 0; it < 2; ++it) r = fma(r, fma(-d, r, 1.0), r);
+    return r;
+}
+
 __device__ __forceinline__ void tsc_cell(double x, double y, int N, double h, double inv_h, int& i, int& j,
                                          double& xl, double& yl) {
     double x_h = div_h(x, h, inv_h) + .5, y_h = div_h(y, h, inv_h) + .5;
@@ -100,9 +132,21 @@ __device__ __forceinline__ void estimate_one(double m, double xi0, double yi0, d
                                              double px, double py, double pz, double dxi, double rb,
                                              double& ex, double& ey) {
     double x = xi0 + xo, y = yi0 + yo;
-    double gamma_m = sqrt(m * m + pz * pz + px * px + py * py);
-    x += px / (gamma_m - pz) * dxi;
-    y += py / (gamma_m - pz) * dxi;
+    const double S = m * m + pz * pz + px * px + py * py;
+    double vx, vy;
+    if (in_fast_range(S)) {
+        double gamma_m, inv;
+        sqrt_fast(S, gamma_m, inv);
+        const double d = gamma_m - pz, r = recip_fast(d);
+        vx = div_h(px, d, r);
+        vy = div_h(py, d, r);
+    } else {
+        const double gamma_m = sqrt(S);
+        vx = px / (gamma_m - pz);
+        vy = py / (gamma_m - pz);
+    }
+    x += vx * dxi;
+    y += vy * dxi;
     if (x >= +rb) x = +2 * rb - x;
     if (x <= -rb) x = -2 * rb - x;
     if (y >= +rb) y = +2 * rb - y;
@@ -132,6 +176,58 @@ __device__ __forceinline__ void store_packed(double* p, double x, double y, doub
     p2[1] = make_double2(m, q);
     p2[2] = make_double2(px, py);
     p2[3] = make_double2(pz, 0.0);
+}
+
+// The momentum push, lcode.py:745-780 (the float64 step kernel of 161^2 spends
+// its time in this chain: 80.1 -> 79.0 us per xi step without the branches, 81^2
+// 74 -> 69, 641^2 363 -> 361): two passes from the old momenta in the
+// gathered fields, then the velocity of the half-way momenta. FAST: without
+// branches (sqrt_fast); returns false if a square root left its range.
+struct Push {
+    double px, py, pz, dpx, dpy, dpz, vx, vy;   // half-way momenta, changes, dx / dxi, dy / dxi
+};
+template <bool FAST>
+__device__ __forceinline__ bool push(double m, double q, double dxi, double opx, double opy, double opz, const double (&F)[6],
+                                     Push& o) {
+    bool ok = true;
+    double px = opx, py = opy, pz = opz;
+#pragma unroll
+    for (int it = 0; it < 3; ++it) {
+        const double S = m * m + pz * pz + px * px + py * py;
+        double gamma_m, inv = 0;
+        if (FAST) {
+            ok = ok && in_fast_range(S);
+            sqrt_fast(S, gamma_m, inv);
+        } else {
+            gamma_m = sqrt(S);
+        }
+        auto over_gamma = [&](double x) { return FAST ? div_h(x, gamma_m, inv) : x / gamma_m; };
+        if (it == 2) {
+            const double d = gamma_m - pz;
+            if (FAST) {
+                const double r = recip_fast(d);
+                o.vx = div_h(px, d, r);
+                o.vy = div_h(py, d, r);
+            } else {
+                o.vx = px / d;
+                o.vy = py / d;
+            }
+            break;
+        }
+        const double vx = over_gamma(px), vy = over_gamma(py), vz = over_gamma(pz);
+        const double d = 1 - vz;
+        const double factor_1 = FAST ? div_h(q * dxi, d, recip_fast(d)) : q * dxi / d;
+        o.dpx = factor_1 * (F[0] + vy * F[5] - vz * F[4]);
+        o.dpy = factor_1 * (F[1] - vx * F[5] + vz * F[3]);
+        o.dpz = factor_1 * (F[2] + vx * F[4] - vy * F[3]);
+        px = opx + o.dpx / 2;
+        py = opy + o.dpy / 2;
+        pz = opz + o.dpz / 2;
+    }
+    o.px = px;
+    o.py = py;
+    o.pz = pz;
+    return ok;
 }
 
 // ---------------------------------------------------------------------------
@@ -174,30 +270,15 @@ __global__ void __launch_bounds__(LC3D_MOVE_THREADS, 1) move_smart_kernel(MoveAr
     double g[6][9];
 #pragma unroll
     for (int f = 0; f < 6; ++f) gather9(a.F[f], t, a.N, g[f]);
-    const double Ex = sum9(g[0], t), Ey = sum9(g[1], t);
-    const double Ez = sum9(g[2], t), Bx = sum9(g[3], t);
-    const double By = sum9(g[4], t), Bz = sum9(g[5], t);
-
-    double px = opx, py = opy, pz = opz;
-    double dpx, dpy, dpz;
+    double F[6];   // Ex Ey Ez Bx By Bz
 #pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        double gamma_m = sqrt(m * m + pz * pz + px * px + py * py);
-        double vx = px / gamma_m, vy = py / gamma_m, vz = pz / gamma_m;
-        double factor_1 = q * a.dxi / (1 - pz / gamma_m);
-        dpx = factor_1 * (Ex + vy * Bz - vz * By);
-        dpy = factor_1 * (Ey - vx * Bz + vz * Bx);
-        dpz = factor_1 * (Ez + vx * By - vy * Bx);
-        px = opx + dpx / 2;
-        py = opy + dpy / 2;
-        pz = opz + dpz / 2;
-    }
-    double gamma_m = sqrt(m * m + pz * pz + px * px + py * py);
-    x_offt += px / (gamma_m - pz) * a.dxi;
-    y_offt += py / (gamma_m - pz) * a.dxi;
-    px = opx + dpx;
-    py = opy + dpy;
-    pz = opz + dpz;
+    for (int f = 0; f < 6; ++f) F[f] = sum9(g[f], t);
+    Push o;
+    if (!push<true>(m, q, a.dxi, opx, opy, opz, F, o)) push<false>(m, q, a.dxi, opx, opy, opz, F, o);
+    x_offt += o.vx * a.dxi;
+    y_offt += o.vy * a.dxi;
+    double px = opx + o.dpx, py = opy + o.dpy;
+    const double pz = opz + o.dpz;
 
     const double rb = a.rb;
     double x = xi0 + x_offt, y = yi0 + y_offt;
@@ -255,39 +336,21 @@ __device__ __forceinline__ void particle_values(FineParticle& p, double m, doubl
     p.djz = pz * dro_g;
 }
 
-// particle_values without branches, so that the chains of a thread's
-// particles overlap (the library's square root and division each end a block
-// of instructions with a test for their slow path: phase 1 of the deposition
-// took 43 of 83 us with them). Goldschmidt's iteration for sqrt(S) and
-// 1 / (2 sqrt(S)), Newton's for the reciprocal of the divisor, from the
-// hardware's approximations; each result is corrected by its exact residual
-// (Markstein), as particle_values' are. Returns false where S is not well
-// inside the range of normal numbers: the caller takes particle_values.
+// particle_values without branches, so that a thread's particles overlap
+// (phase 1 of the deposition took 43 of 83 us with the library's functions).
+// Returns false where the caller has to take particle_values.
 __device__ __forceinline__ bool particle_values_fast(FineParticle& p, double m, double q, double px, double py,
                                                      double pz) {
     const double S = m * m + px * px + py * py + pz * pz;
-    double y, r;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(S));
-    double g = S * y, h = .5 * y;
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const double e = fma(-g, h, .5);
-        g = fma(g, e, g);
-        h = fma(h, e, h);
-    }
-    g = fma(fma(-g, g, S), h, g);
-    double inv = h + h;
-    inv = fma(inv, fma(-g, inv, 1.0), inv);
+    double g, inv;
+    sqrt_fast(S, g, inv);
     const double d = 1 - div_h(pz, g, inv);
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-#pragma unroll
-    for (int it = 0; it < 2; ++it) r = fma(r, fma(-d, r, 1.0), r);
-    p.dro = div_h(q, d, r);
+    p.dro = div_h(q, d, recip_fast(d));
     const double dro_g = div_h(p.dro, g, inv);
     p.djx = px * dro_g;
     p.djy = py * dro_g;
     p.djz = pz * dro_g;
-    return S > 0x1p-900 && S < 0x1p900;
+    return in_fast_range(S);
 }
 
 // The cell of one coordinate and the offset from its centre (tsc_cell): the

@@ -354,7 +354,7 @@ int run_step(lc3d_ctx* c, const lc3d_state_ptrs& prev, const lc3d_state_ptrs& ou
             so.out[0] = out.Ex; so.out[1] = out.Ey; so.out[2] = out.Ez;
             so.out[3] = out.Bx; so.out[4] = out.By; so.out[5] = out.Bz;
         }
-        if (x && x->beam_host) LC3D_CUDA_TRY(cudaStreamWaitEvent(s, c->ev_copy, 0));
+        if (pass == 0 && x && x->beam_host) LC3D_CUDA_TRY(cudaStreamWaitEvent(s, c->ev_copy, 0));
         LC3D_TRY(solve_fields(c, LC3D_F_ALL, in, so, s));
     }
     if (predicted && x->residual) {

@@ -7,7 +7,7 @@
 //     rho_b = A exp(-(x^2 + y^2) / (2 sigma_r^2)) 0.5 (1 - cos(sqrt(pi/2) xi / L))
 // for 0 <= xi <= 2 sqrt(2 pi) L (else 0), xi = xi_i xi_step_size, is evaluated
 // by a kernel from a device xi counter, and Ez at the grid centre is appended
-// to a device array after every step. One whole xi step (beam, the 23 solver
+// to a device array after every step. One whole xi step (beam, the solver's
 // launches, the record) is captured once per state parity into a CUDA graph
 // and replayed.
 

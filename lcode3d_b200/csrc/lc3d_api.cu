@@ -121,13 +121,36 @@ __global__ void __launch_bounds__(256) copy_state_kernel(const __grid_constant__
     }
 }
 
-int copy_state(const lc3d_state_ptrs& dst, const lc3d_state_ptrs& src, size_t np, size_t ng, cudaStream_t s) {
+// Whether a kernel on `device` may access p: its own memory or managed
+// memory. The runtime copies from and to other memory (a peer's), or refuses
+// the pointer, which a kernel cannot.
+bool on_device(const void* p, int device) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return (at.type == cudaMemoryTypeDevice && at.device == device) || at.type == cudaMemoryTypeManaged;
+}
+
+int copy_state(const lc3d_state_ptrs& dst, const lc3d_state_ptrs& src, size_t np, size_t ng, const lc3d_ctx* c,
+               const lc3d_state_ptrs& caller, cudaStream_t s) {
     const CopyArgs a = {{dst.x_offt, dst.y_offt, dst.px, dst.py, dst.pz, dst.Ex, dst.Ey, dst.Ez,
                          dst.Bx, dst.By, dst.Bz, dst.ro, dst.jx, dst.jy, dst.jz},
                         {src.x_offt, src.y_offt, src.px, src.py, src.pz, src.Ex, src.Ey, src.Ez,
                          src.Bx, src.By, src.Bz, src.ro, src.jx, src.jy, src.jz}, np, ng};
     for (int k = 0; k < 15; ++k)
         if (!a.dst[k] || !a.src[k]) return LC3D_ERR_PARAM;
+    double* const theirs[] = {caller.x_offt, caller.y_offt, caller.px, caller.py, caller.pz, caller.Ex, caller.Ey, caller.Ez,
+                              caller.Bx, caller.By, caller.Bz, caller.ro, caller.jx, caller.jy, caller.jz};
+    bool own = true;
+    for (double* q : theirs) own = own && on_device(q, c->device);
+    if (!own) {
+        for (int k = 0; k < 15; ++k)
+            LC3D_CUDA_TRY(cudaMemcpyAsync(a.dst[k], a.src[k], (k < 5 ? np : ng) * sizeof(double),
+                                          cudaMemcpyDeviceToDevice, s));
+        return LC3D_OK;
+    }
     const unsigned blocks = (unsigned)((ng / 2 + 255) / 256);
     copy_state_kernel<<<dim3(blocks < 1 ? 1 : blocks > 296 ? 296 : blocks, 15), 256, 0, s>>>(a);
     LC3D_CUDA_TRY(cudaGetLastError());
@@ -776,7 +799,7 @@ int lc3d_get_const(lc3d_ctx* c, double* m, double* q, double* x_init, double* y_
 int lc3d_set_state(lc3d_ctx* c, const lc3d_state_ptrs* s, void* stream) {
     if (!c || !state_complete(s)) return LC3D_ERR_PARAM;
     DeviceGuard g(c->device);
-    LC3D_TRY(copy_state(c->st[c->cur], *s, (size_t)c->Nc * c->Nc, (size_t)c->N * c->N, S(stream)));
+    LC3D_TRY(copy_state(c->st[c->cur], *s, (size_t)c->Nc * c->Nc, (size_t)c->N * c->N, c, *s, S(stream)));
     c->state_set = 1;
     return LC3D_OK;
 }
@@ -785,7 +808,7 @@ int lc3d_get_state(lc3d_ctx* c, lc3d_state_ptrs* s, void* stream) {
     if (!c || !state_complete(s)) return LC3D_ERR_PARAM;
     if (!c->state_set) return LC3D_ERR_STATE;
     DeviceGuard g(c->device);
-    return copy_state(*s, c->st[c->cur], (size_t)c->Nc * c->Nc, (size_t)c->N * c->N, S(stream));
+    return copy_state(*s, c->st[c->cur], (size_t)c->Nc * c->Nc, (size_t)c->N * c->N, c, *s, S(stream));
 }
 
 int lc3d_step(lc3d_ctx* c, const double* beam_ro, void* stream) {

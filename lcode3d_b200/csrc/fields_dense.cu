@@ -33,6 +33,13 @@ struct FoldArgs {
     int rows[6], cols[6];
 };
 
+// A folded row: the even part, then the odd part from the next 128-byte line
+// on. Every operand of the GEMMs (folded planes, their odd parts, the half
+// matrices) has its rows on whole lines, so that copies of 16 bytes apply and
+// a k-step of 16 touches one line per row.
+__host__ __device__ constexpr int odd_at(int n) { return (n / 2 + 16) & ~15; }          // n odd
+__host__ __device__ constexpr int folded_width(int n) { return odd_at(n) + n / 2; }
+
 // One thread per (a, b), a <= (rows - 1) / 2, b <= (cols - 1) / 2 (sizes are
 // odd): the four cells it mirrors to, and the four sums and differences. The
 // centre is its own mirror and belongs to the even part alone.
@@ -49,10 +56,11 @@ __global__ void __launch_bounds__(128) fold_kernel(const __grid_constant__ FoldA
     const double x11 = a < c0 && b < c1 ? x[(size_t)a2 * g.ld_in + b2] : 0.0;
     double* o = g.out[f];
     const size_t even = (size_t)a * g.ld_out, odd = (size_t)(c0 + 1 + a) * g.ld_out;
+    const int b1 = odd_at(g.cols[f]) + b;
     o[even + b] = (x00 + x01) + (x10 + x11);
-    if (b < c1) o[even + c1 + 1 + b] = (x00 - x01) + (x10 - x11);
+    if (b < c1) o[even + b1] = (x00 - x01) + (x10 - x11);
     if (a < c0) o[odd + b] = (x00 + x01) - (x10 + x11);
-    if (a < c0 && b < c1) o[odd + c1 + 1 + b] = (x00 - x01) - (x10 - x11);
+    if (a < c0 && b < c1) o[odd + b1] = (x00 - x01) - (x10 - x11);
 }
 
 // The inverse walk: value and mirrors from the even and odd parts.
@@ -64,10 +72,11 @@ __global__ void __launch_bounds__(128) unfold_kernel(const __grid_constant__ Fol
     const int a2 = g.rows[f] - 1 - a, b2 = g.cols[f] - 1 - b;
     const double* x = g.in[f];
     const size_t even = (size_t)a * g.ld_in, odd = (size_t)(c0 + 1 + a) * g.ld_in;
+    const int b1 = odd_at(g.cols[f]) + b;
     const double ee = x[even + b];
-    const double eo = b < c1 ? x[even + c1 + 1 + b] : 0.0;
+    const double eo = b < c1 ? x[even + b1] : 0.0;
     const double oe = a < c0 ? x[odd + b] : 0.0;
-    const double oo = a < c0 && b < c1 ? x[odd + c1 + 1 + b] : 0.0;
+    const double oo = a < c0 && b < c1 ? x[odd + b1] : 0.0;
     double* o = g.out[f];
     o[(size_t)a * g.ld_out + b] = (ee + eo) + (oe + oo);
     if (b < c1) o[(size_t)a * g.ld_out + b2] = (ee - eo) + (oe - oo);
@@ -75,29 +84,36 @@ __global__ void __launch_bounds__(128) unfold_kernel(const __grid_constant__ Fol
     if (a < c0 && b < c1) o[(size_t)a2 * g.ld_out + b2] = (ee - eo) - (oe - oo);
 }
 
-// out[i][j] = lam[k0 of i][k1 of j], both axes sorted by parity.
+// out[i][j] = lam[k0 of i][k1 of j], both axes sorted by parity, the columns
+// as a folded row's (0 between the parts).
 __global__ void lam_parity_kernel(const double* __restrict__ lam, int rows, int cols, double* __restrict__ out) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
-    if (j >= cols) return;
-    const int e0 = (rows + 1) / 2, e1 = (cols + 1) / 2;
-    const int k0 = i < e0 ? 2 * i : 2 * (i - e0) + 1, k1 = j < e1 ? 2 * j : 2 * (j - e1) + 1;
-    out[(size_t)i * cols + j] = lam[(size_t)k0 * cols + k1];
+    const int width = folded_width(cols), j1 = odd_at(cols);
+    if (j >= width) return;
+    const int e0 = (rows + 1) / 2;
+    const int k0 = i < e0 ? 2 * i : 2 * (i - e0) + 1, k1 = j < j1 ? 2 * j : 2 * (j - j1) + 1;
+    out[(size_t)i * width + j] = k1 < cols ? lam[(size_t)k0 * cols + k1] : 0.0;
 }
 
 // ---------------------------------------------------------------------------
 // Batched float64 GEMM, C = A B (optionally C = Lambda o (A B)), row-major,
 // on the float64 tensor cores (mma.sync m16n8k8 .f64: float64 products and
 // sums throughout). 64 x 32 tiles per 64-thread CTA, a 32 x 32 tile (2 x 4
-// MMAs per k8 step) per warp; k-steps of 16 staged by
-// cp.async into two shared-memory buffers, the next k-step copied while the
-// current one is multiplied.
+// MMAs per k8 step) per warp; k-steps of 16 staged by 16-byte cp.async into
+// two shared-memory buffers, the next k-step copied while the current one is
+// multiplied. With copies of 8 bytes, twice as many and each with its address
+// arithmetic, the MMA pipe was 53 % busy; with these an xi step in a
+// graph at 255^2 172 -> 157 us, 387^2 316 -> 292, 641^2 970 -> 911 (rows on 16
+// bytes only 162, 301, 920; past L1, as .cg, 163, 394, 910: the CTAs of an SM
+// share their panels there).
 //
 // The tile is small because the problems are: at 387^2 a launch has 12 of
 // about 387 x 194 x 194, and what is lost is rows and columns past the edges
-// and SMs with a tile less than others. 28 us a launch at 387^2 (two or three
-// 64 x 32 tiles' k-steps in flight per scheduler; 35 with m8n8k4 MMAs and
-// bounds checks on every copy); 78 with matrices of full size in 128 x 64
-// tiles.
+// and SMs with a tile less than others. 28 us a launch at 387^2 with 8-byte copies
+// (two or three 64 x 32 tiles' k-steps in flight per scheduler), some 25 now;
+// 35 with m8n8k4 MMAs and bounds checks on every copy; 78 with matrices of
+// full size in 128 x 64 tiles. Leaving out the MMAs past the edges (a fifth
+// of a launch's at 387^2) was slower: 316 -> 340, for the branches.
 // ---------------------------------------------------------------------------
 constexpr int MAX_PROBS = 12;
 
@@ -122,9 +138,9 @@ constexpr int AS_LD = GK + 4;    // As[m][k]
 constexpr int BS_LD = GTN + 4;   // Bs[k][n]
 constexpr int AS_SIZE = GTM * AS_LD, BS_SIZE = GK * BS_LD;
 
-// 8-byte global -> shared copy; a source size of 0 writes zeros.
-__device__ __forceinline__ void cp_async8(uint32_t dst, const double* src, int size) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
+// 16-byte global -> shared copy; zeros past the source size.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const double* src, int size) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
 }
 
 // c += a b, 16 x 8 x 8. Thread (g, t) = (lane / 4, lane % 4) holds a[i] at
@@ -153,29 +169,30 @@ __global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_con
     const int wm = warp % (GTM / 32) * 32, wn = warp / (GTM / 32) * 32;
     pdl_wait();
 
-    // Rows of A past M and columns of B past N repeat the last one (nothing of
+    // Rows of A past M and columns of B past N repeat the last ones (nothing of
     // them is stored), so a copy's address costs a clamp and a multiply; past
-    // K zeros are copied. A: 4 rows x 16 k per pass of the threads; B: 2 k
-    // rows x 32 columns.
+    // K zeros are copied. Rows start on 16 bytes at an even pitch, so a copy
+    // of two columns that starts inside a row stays inside it. A: 8 rows x 16 k per
+    // pass of the threads; B: 4 k rows x 32 columns.
     static_assert(GEMM_THREADS == 64 && GK == 16 && GTN == 32, "the copies' shapes");
-    const int ra = tid / GK, ka = tid % GK, kb = tid / GTN, nb = tid % GTN;
-    const int alast = P.M - 1 - row0 - ra, astep = 4;
+    const int ra = tid >> 3, ka = (tid & 7) * 2, kb = tid >> 4, nb = (tid & 15) * 2;
+    const int alast = P.M - 1 - row0 - ra;
     const double* pa = P.A + (size_t)(row0 + ra) * P.lda + ka;
-    const double* pb = P.B + (size_t)kb * P.ldb + min(col0 + nb, P.N - 1);
+    const double* pb = P.B + (size_t)kb * P.ldb + min(col0 + nb, (P.N - 1) & ~1);
     const uint32_t sa = static_cast<uint32_t>(__cvta_generic_to_shared(As + ra * AS_LD + ka));
     const uint32_t sb = static_cast<uint32_t>(__cvta_generic_to_shared(Bs + kb * BS_LD + nb));
     auto load = [&](int k0, int buf) {
-        const int size_a = k0 + ka < P.K ? 8 : 0;
+        const int size_a = max(0, min(2, P.K - k0 - ka)) * 8;
         const double* a = size_a ? pa + k0 : P.A;
         const int lda = size_a ? P.lda : 0;
 #pragma unroll
-        for (int i = 0; i < GTM / astep; ++i)
-            cp_async8(sa + (buf * AS_SIZE + i * astep * AS_LD) * 8, a + (ptrdiff_t)min(i * astep, alast) * lda, size_a);
+        for (int i = 0; i < GTM / 8; ++i)
+            cp_async16(sa + (buf * AS_SIZE + i * 8 * AS_LD) * 8, a + (ptrdiff_t)min(i * 8, alast) * lda, size_a);
         const double* b = pb + (size_t)k0 * P.ldb;
 #pragma unroll
-        for (int i = 0; i < GK / 2; ++i) {
-            const bool in = k0 + kb + 2 * i < P.K;
-            cp_async8(sb + (buf * BS_SIZE + i * 2 * BS_LD) * 8, in ? b + (ptrdiff_t)(2 * i) * P.ldb : P.B, in ? 8 : 0);
+        for (int i = 0; i < GK / 4; ++i) {
+            const bool in = k0 + kb + 4 * i < P.K;
+            cp_async16(sb + (buf * BS_SIZE + i * 4 * BS_LD) * 8, in ? b + (ptrdiff_t)(4 * i) * P.ldb : P.B, in ? 16 : 0);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -264,7 +281,7 @@ double sin_pi_frac(long long r, long long L) {
 
 // Half-size matrices of a transform type, by parity q (0 even, 1 odd) of the
 // frequency: forth[k][n] = T[2 k + q][n], back[n][k] = T[n][2 k + q], and
-// their transposes, all n_q x n_q.
+// their transposes, all n_q x n_q at a pitch of whole lines.
 struct HalfMats {
     double *forth, *forth_t, *back, *back_t;
 };
@@ -276,6 +293,8 @@ struct DenseState {
 
 // Size of parity q's half of a transform of `n` points (odd).
 int half(int n, int q) { return q ? n / 2 : n / 2 + 1; }
+
+int mat_pitch(int n) { return (n + 15) & ~15; }
 
 }  // namespace
 
@@ -294,15 +313,16 @@ int dense_init(lc3d_ctx* c) {
                 const long long r = (k * x) % (2 * L);
                 return (x == 0 || x == L ? 1.0 : 2.0) * sin_pi_frac(2 * r + L, 2 * L);
             };
-            const size_t nn = (size_t)n * n;
-            std::vector<double> h(4 * nn);
+            const int ld = mat_pitch(n);
+            const size_t nn = (size_t)n * ld;
+            std::vector<double> h(4 * nn, 0.0);
             for (int k = 0; k < n; ++k)
                 for (int x = 0; x < n; ++x) {
                     const double f = T(2 * k + q, x), b = T(x, 2 * k + q);
-                    h[(size_t)k * n + x] = f;
-                    h[nn + (size_t)x * n + k] = f;
-                    h[2 * nn + (size_t)x * n + k] = b;
-                    h[3 * nn + (size_t)k * n + x] = b;
+                    h[(size_t)k * ld + x] = f;
+                    h[nn + (size_t)x * ld + k] = f;
+                    h[2 * nn + (size_t)x * ld + k] = b;
+                    h[3 * nn + (size_t)k * ld + x] = b;
                 }
             HalfMats& m = d->m[type][q];
             LC3D_CUDA_TRY(cudaMalloc(&m.forth, 4 * nn * sizeof(double)));
@@ -314,8 +334,9 @@ int dense_init(lc3d_ctx* c) {
     const double* src[4] = {c->lam_neu, c->lam_mixT, c->lam_mix, c->lam_dir};
     for (int k = 0; k < 4; ++k) {
         const int rows = N - 2 * (k >> 1), cols = N - 2 * (k & 1);
-        LC3D_CUDA_TRY(cudaMalloc(&d->lam[k], (size_t)rows * cols * sizeof(double)));
-        lam_parity_kernel<<<dim3((cols + 127) / 128, rows), 128>>>(src[k], rows, cols, d->lam[k]);
+        const int width = folded_width(cols);
+        LC3D_CUDA_TRY(cudaMalloc(&d->lam[k], (size_t)rows * width * sizeof(double)));
+        lam_parity_kernel<<<dim3((width + 127) / 128, rows), 128>>>(src[k], rows, cols, d->lam[k]);
         LC3D_CUDA_TRY(cudaGetLastError());
     }
     return LC3D_OK;
@@ -335,10 +356,11 @@ void dense_free(lc3d_ctx* c) {
 
 int dense_solve(lc3d_ctx* c, const DenseDesc* desc, int count, cudaStream_t s) {
     const DenseState* d = static_cast<const DenseState*>(c->dense);
-    const int N = c->N;
+    const int N = c->N, ld = fft64_pitch(N);   // t1, t2: rows on whole lines
     const dim3 fold_grid(((N + 1) / 2 + 127) / 128, (N + 1) / 2, count);
     FoldArgs fa{};
-    fa.ld_in = fa.ld_out = N;
+    fa.ld_in = N;
+    fa.ld_out = ld;
     for (int f = 0; f < count; ++f) {
         fa.rows[f] = N - 2 * desc[f].type0;
         fa.cols[f] = N - 2 * desc[f].type1;
@@ -362,28 +384,30 @@ int dense_solve(lc3d_ctx* c, const DenseDesc* desc, int count, cudaStream_t s) {
                 const double* in = right ? e.t2 : e.t1;
                 double* out = right ? e.t1 : e.t2;
                 if (right) {        // columns of parity q
-                    const int n = half(cols, q), at = q * half(cols, 0);
+                    const int n = half(cols, q), at = q * odd_at(cols);
                     const HalfMats& m = d->m[e.type1][q];
-                    p.A = in + at; p.lda = N;
-                    p.B = back ? m.back_t : m.forth_t; p.ldb = n;
-                    p.C = out + at; p.ldc = N;
+                    p.A = in + at; p.lda = ld;
+                    p.B = back ? m.back_t : m.forth_t; p.ldb = mat_pitch(n);
+                    p.C = out + at; p.ldc = ld;
                     p.M = rows; p.N = n; p.K = n;
                 } else {            // rows of parity q
                     const int n = half(rows, q), at = q * half(rows, 0);
                     const HalfMats& m = d->m[e.type0][q];
-                    p.A = back ? m.back : m.forth; p.lda = n;
-                    p.B = in + (size_t)at * N; p.ldb = N;
-                    p.C = out + (size_t)at * N; p.ldc = N;
-                    p.M = n; p.N = cols; p.K = n;
+                    p.A = back ? m.back : m.forth; p.lda = mat_pitch(n);
+                    p.B = in + (size_t)at * ld; p.ldb = ld;
+                    p.C = out + (size_t)at * ld; p.ldc = ld;
+                    p.M = n; p.N = folded_width(cols); p.K = n;
                     if (!back) {
-                        p.L = d->lam[e.type0 * 2 + e.type1] + (size_t)at * cols;
-                        p.ldl = cols;
+                        p.L = d->lam[e.type0 * 2 + e.type1] + (size_t)at * p.N;
+                        p.ldl = p.N;
                     }
                 }
             }
         }
         LC3D_TRY(launch_gemm(c, b, s));
     }
+    fa.ld_in = ld;
+    fa.ld_out = N;
     for (int f = 0; f < count; ++f) {
         fa.in[f] = desc[f].t2;
         fa.out[f] = desc[f].out;

@@ -98,7 +98,7 @@ __global__ void lam_parity_kernel(const double* __restrict__ lam, int rows, int 
 // ---------------------------------------------------------------------------
 // Batched float64 GEMM, C = A B (optionally C = Lambda o (A B)), row-major,
 // on the float64 tensor cores (mma.sync m16n8k8 .f64: float64 products and
-// sums throughout). 64 x 32 tiles per 64-thread CTA, a 32 x 32 tile (2 x 4
+// sums throughout). 64 x 32 tiles per 128-thread CTA, a 32 x 16 tile (2 x 2
 // MMAs per k8 step) per warp; k-steps of 16 staged by 16-byte cp.async into
 // two shared-memory buffers, the next k-step copied while the current one is
 // multiplied. With copies of 8 bytes, twice as many and each with its address
@@ -110,10 +110,15 @@ __global__ void lam_parity_kernel(const double* __restrict__ lam, int rows, int 
 // The tile is small because the problems are: at 387^2 a launch has 12 of
 // about 387 x 194 x 194, and what is lost is rows and columns past the edges
 // and SMs with a tile less than others. 28 us a launch at 387^2 with 8-byte copies
-// (two or three 64 x 32 tiles' k-steps in flight per scheduler), some 25 now;
-// 35 with m8n8k4 MMAs and bounds checks on every copy; 78 with matrices of
-// full size in 128 x 64 tiles. Leaving out the MMAs past the edges (a fifth
-// of a launch's at 387^2) was slower: 316 -> 340, for the branches.
+// and two warps of 32 x 32; 35 with m8n8k4 MMAs and bounds checks on every
+// copy; 78 with matrices of full size in 128 x 64 tiles. Four warps of 32 x 16
+// a CTA hide more of a k-step's latency than two of 32 x 32 (an xi step in a
+// graph at 43^2 91 -> 80 us, 163^2 128 -> 107, 255^2 157 -> 142, 431^2 370 ->
+// 350, 513^2 495 -> 482, 641^2 911 -> 772; 387^2 292 -> 297); five CTAs per SM
+// instead of six 524 at 513^2. Leaving out the MMAs past the edges (a fifth
+// of a launch's at 387^2) was slower, for the branches: 316 -> 340; whole
+// warps left out changed nothing. Tiles of 32 x 64 where they are fewer: 431^2
+// 350 -> 340, but 387^2 297 -> 301.
 // ---------------------------------------------------------------------------
 constexpr int MAX_PROBS = 12;
 
@@ -130,7 +135,8 @@ struct GemmBatch {
 };
 
 constexpr int GTM = 64, GTN = 32, GK = 16;
-constexpr int GEMM_THREADS = GTM / 32 * (GTN / 32) * 32;
+constexpr int GWN = 16;          // columns per warp
+constexpr int GEMM_THREADS = GTM / 32 * (GTN / GWN) * 32;
 // shared pitches (doubles): the fragment loads of a half-warp (rows g = 0..3
 // or 4..7, columns t = 0..3) fall in distinct banks: 2 (20 g + t) and
 // 2 (36 t + g) mod 32 are distinct over the 16 lanes
@@ -153,7 +159,7 @@ __device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], const
         : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-__global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_constant__ GemmBatch b) {
+__global__ void __launch_bounds__(GEMM_THREADS, 6) dgemm_kernel(const __grid_constant__ GemmBatch b) {
     __shared__ __align__(16) double As[2 * AS_SIZE], Bs[2 * BS_SIZE];
     const int bid = blockIdx.x;
     int pi = 0;
@@ -166,15 +172,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_con
     const int row0 = tm * GTM, col0 = tn * GTN;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tq = lane & 3;            // fragment row group, thread in group
-    const int wm = warp % (GTM / 32) * 32, wn = warp / (GTM / 32) * 32;
+    const int wm = warp % (GTM / 32) * 32, wn = warp / (GTM / 32) * GWN;
     pdl_wait();
 
     // Rows of A past M and columns of B past N repeat the last ones (nothing of
     // them is stored), so a copy's address costs a clamp and a multiply; past
     // K zeros are copied. Rows start on 16 bytes at an even pitch, so a copy
-    // of two columns that starts inside a row stays inside it. A: 8 rows x 16 k per
-    // pass of the threads; B: 4 k rows x 32 columns.
-    static_assert(GEMM_THREADS == 64 && GK == 16 && GTN == 32, "the copies' shapes");
+    // of two columns that starts inside a row stays inside it. A: 16 rows x 16 k
+    // per pass of the threads; B: 8 k rows x 32 columns.
+    static_assert(GEMM_THREADS == 128 && GK == 16 && GTN == 32, "the copies' shapes");
     const int ra = tid >> 3, ka = (tid & 7) * 2, kb = tid >> 4, nb = (tid & 15) * 2;
     const int alast = P.M - 1 - row0 - ra;
     const double* pa = P.A + (size_t)(row0 + ra) * P.lda + ka;
@@ -186,22 +192,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_con
         const double* a = size_a ? pa + k0 : P.A;
         const int lda = size_a ? P.lda : 0;
 #pragma unroll
-        for (int i = 0; i < GTM / 8; ++i)
-            cp_async16(sa + (buf * AS_SIZE + i * 8 * AS_LD) * 8, a + (ptrdiff_t)min(i * 8, alast) * lda, size_a);
+        for (int i = 0; i < GTM / 16; ++i)
+            cp_async16(sa + (buf * AS_SIZE + i * 16 * AS_LD) * 8, a + (ptrdiff_t)min(i * 16, alast) * lda, size_a);
         const double* b = pb + (size_t)k0 * P.ldb;
 #pragma unroll
-        for (int i = 0; i < GK / 4; ++i) {
-            const bool in = k0 + kb + 4 * i < P.K;
-            cp_async16(sb + (buf * BS_SIZE + i * 4 * BS_LD) * 8, in ? b + (ptrdiff_t)(4 * i) * P.ldb : P.B, in ? 16 : 0);
+        for (int i = 0; i < GK / 8; ++i) {
+            const bool in = k0 + kb + 8 * i < P.K;
+            cp_async16(sb + (buf * BS_SIZE + i * 8 * BS_LD) * 8, in ? b + (ptrdiff_t)(8 * i) * P.ldb : P.B, in ? 16 : 0);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    double acc[2][4][4];
+    double acc[2][GWN / 8][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < GWN / 8; ++j)
 #pragma unroll
             for (int h = 0; h < 4; ++h) acc[i][j][h] = 0.0;
 
@@ -215,19 +221,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_con
         const double* bs = Bs + (kt & 1) * BS_SIZE + tq * BS_LD + wn + g;
 #pragma unroll
         for (int ks = 0; ks < GK; ks += 8) {
-            double af[2][4], bf[4][2];
+            double af[2][4], bf[GWN / 8][2];
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
                 for (int h = 0; h < 4; ++h) af[i][h] = as[(i * 16 + (h & 1) * 8) * AS_LD + ks + (h >> 1) * 4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < GWN / 8; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) bf[j][h] = bs[(ks + h * 4) * BS_LD + j * 8];
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dmma(acc[i][j], af[i], bf[j]);
+                for (int j = 0; j < GWN / 8; ++j) dmma(acc[i][j], af[i], bf[j]);
         }
     }
     // accumulator (i, j, h): row wm + 16 i + g + 8 (h >> 1), column wn + 8 j +
@@ -236,15 +242,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 7) dgemm_kernel(const __grid_con
     for (int i = 0; i < 4; ++i) {
         const int row = row0 + wm + 8 * i + g, c0 = col0 + wn + 2 * tq;
         if (row >= P.M) continue;
-        double l[8];
+        double l[GWN / 4];
         if (P.L)
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < GWN / 4; ++u) {
                 const int col = c0 + u / 2 * 8 + u % 2;
                 l[u] = col < P.N ? __ldg(P.L + (size_t)row * P.ldl + col) : 0.0;
             }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < GWN / 4; ++u) {
             const int col = c0 + u / 2 * 8 + u % 2;
             if (col >= P.N) continue;
             double v = acc[i >> 1][u / 2][(i & 1) * 2 + u % 2];

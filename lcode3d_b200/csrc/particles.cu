@@ -651,6 +651,10 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
     imax = __reduce_max_sync(0xffffffffu, imax);
     jmin = __reduce_min_sync(0xffffffffu, jmin);
     jmax = __reduce_max_sync(0xffffffffu, jmax);
+    // thread 0's empty bounding box is there before any warp adds to it. Here,
+    // beside the next barrier, where the warps wait for the last one's phase 1
+    // anyway
+    __syncthreads();
     if (lane == 0 && imin <= imax) {
         atomicMin(&s_bb[0], imin);
         atomicMax(&s_bb[1], imax);

@@ -289,8 +289,9 @@ int lc3d_check_error(lc3d_ctx* ctx, void* stream);
 
 /* Tile shapes of this context (no reference counterpart; the autotuner of
  * lcode3d_b200.batch picks them per grid size). deposit_rows: fine-lattice
- * rows per CTA of the deposition, 4, 8 or 16 (0: the default, 12); the CTA
- * covers that many rows x 32 columns.
+ * rows per CTA of the deposition, 4, 8 or 16; the CTA covers that many rows
+ * x 32 columns. 0: the default, 12 rows, or on small lattices (up to 240
+ * fine particles a side at fineness 2, 400 at others) 4 rows, a warp for each.
  * fft_ctas_per_sm: resident CTAs per SM of the persistent float32 FFT row
  * passes (0: as many as fit; the float64 FFT kernels are not persistent and
  * take no setting). Results agree to rounding (the deposition's window

@@ -189,6 +189,7 @@ DepositArgs deposit_args(lc3d_ctx* c, int buf, const double* x, const double* y,
     a.acc = c->acc[buf];
     a.plane = c->acc_plane;
     a.Nc = c->Nc; a.Nf = c->Nf; a.N = c->N;
+    a.fineness = c->p.plasma_fineness;
     a.fine_off = deposit_fine_offset(c->p.plasma_fineness);
     a.tile_rows = c->dep_rows;
     a.h = c->p.grid_step_size; a.inv_h = 1.0 / c->p.grid_step_size; a.sf = c->sf;

@@ -103,9 +103,9 @@ struct DepositArgs {
     const double* packed;                                     // optional: the 7 coarse arrays as [Nc*Nc][8]
     unsigned long long* acc;                                  // 8 planes of fixed-point words
     size_t plane;                                             // plane stride (>= N*N, 256-byte multiple)
-    int Nc, Nf, N;
+    int Nc, Nf, N, fineness;
     int fine_off;                                             // tile origin: fine_off particles before 0
-    int tile_rows;                                            // fine rows per CTA (4, 8, 12, 16; 0: default)
+    int tile_rows;                                            // fine rows per CTA (4, 8, 16; 0: by the lattice's size)
     double h, inv_h, sf;
     unsigned* err;
 };
@@ -130,16 +130,15 @@ int launch_move_estimate(const EstimateArgs& a, cudaStream_t s);
 int launch_move_smart(const MoveArgs& a, cudaStream_t s);
 int launch_deposit_main(const DepositArgs& a, cudaStream_t s);
 int deposit_fine_offset(int fineness);
-// Default fine rows per deposition CTA (4, 8, 12 or 16: dep_threads).
+// Fine rows per deposition CTA where neither a tile setting nor the rule for
+// small lattices says otherwise (particles.cu: dep_threads, dep_small).
 #ifndef LC3D_DEP_ROWS
 #define LC3D_DEP_ROWS 12
 #endif
-// Depositions of several simulations in one launch (batches): tiles of
-// DEP_MULTI_ROWS fine rows, CTA b of the launch takes tile b - cta_start[s]
-// of simulation s. The same height as the default: the window's float64 sums
-// follow the tile, so only the same tiles give results bit-identical to each
-// simulation run alone.
-constexpr int DEP_MULTI_ROWS = LC3D_DEP_ROWS;
+// Depositions of several simulations in one launch (batches): CTA b of the
+// launch takes tile b - cta_start[s] of simulation s. The tiles are the
+// default ones: the window's float64 sums follow the tile, so only the same
+// tiles give results bit-identical to each simulation run alone.
 int deposit_multi_tiles(const DepositArgs& a);
 int launch_deposit_multi(const DepositArgs* args_dev, const int* cta_start_dev, int n, int ctas, cudaStream_t s);
 int launch_deposit_finalize(const DepositFinalizeArgs& f, cudaStream_t s);

@@ -409,8 +409,8 @@ __device__ __forceinline__ void fx_add(unsigned long long* hi_plane, unsigned lo
 
 // ---------------------------------------------------------------------------
 // Deposition kernel. A CTA deposits a tile of TI fine-lattice rows x 32
-// columns, three rows per warp.
-//  1. Three fine particles per thread, one per row of its warp. Coarse->fine
+// columns, three rows per warp (one on small lattices).
+//  1. As many fine particles per thread, one per row of its warp. Coarse->fine
 //     mix in two separable passes (the equivalent formula noted beside the
 //     reference's make_plasma, lcode.py:554-556): the warp first mixes the two
 //     coarse rows of each fine row fi,
@@ -423,7 +423,8 @@ __device__ __forceinline__ void fx_add(unsigned long long* hi_plane, unsigned lo
 //     global memory (fine_particle). Then the deposit values
 //     (lcode.py:651-655) and the TSC cell; cell offsets and values are staged
 //     in shared memory.
-//  2. One thread per cell. Every particle sets its bit in its cell's masks
+//  2. One thread per cell (two or four with the fields split between them on
+//     small lattices). Every particle sets its bit in its cell's masks
 //     (one word per fine row, one bit per column), so a cell's thread meets
 //     its particles in the order of the lattice, whatever the timing. It sums
 //     their stencils, all four fields, into a 3 x 3 patch in registers: the
@@ -451,18 +452,41 @@ __device__ __forceinline__ void fx_add(unsigned long long* hi_plane, unsigned lo
 // against 66.
 // ---------------------------------------------------------------------------
 constexpr int DEP_TW = 32;                  // fine columns of a tile, one per lane
-constexpr int DEP_RPW = 3;                  // fine rows per warp
 constexpr int DEP_CMAX = 16;                // coarse columns the row tables hold
 constexpr int DEP_CELLS = 256;              // cells with particles in a window
 constexpr int DEP_SIDE = 32;                // ... their rows or columns at most
 constexpr int DEP_STRIPS = 4;               // windows of a tile, one after the other (rarefied plasma)
 constexpr int DEP_WIN = 352;                // window cells, (rows + 2) (columns + 2) <= 340
 
-// Threads of a tile of `ti` rows. 12 rows: 384 particles on 128 threads, and
-// at most 7 x 17 cells of an undisturbed lattice, one round of the threads (us
-// per xi step with 12 / 4 / 8 / 16 rows: 641^2 367 / 419 / 375 / 402, 321^2
-// 132 / 160 / 137 / 138, 161^2 86.5 / 86.1 / 83.2 / 84.3).
-__host__ __device__ constexpr int dep_threads(int ti) { return (ti + DEP_RPW - 1) / DEP_RPW * 32; }
+// Threads of a tile of `ti` rows, `rpw` of them per warp. 12 rows, three per
+// warp: 384 particles on 128 threads, and at most 7 x 17 cells of an
+// undisturbed lattice, one round of the threads (us per deposition with its
+// finalize, 12 / 4 / 8 / 16 rows, plasma displaced by several cells: 641^2
+// 69.5 / 93.5 / 76.6 / 85.4, 321^2 21.6 / 26.7 / 22.4 / 25.8).
+__host__ __device__ constexpr int dep_threads(int ti, int rpw = 3) { return (ti + rpw - 1) / rpw * 32; }
+
+// A lattice of few tiles leaves most of the chip idle, and what counts is how
+// long one tile takes: four rows, one per warp (a row's particles are a chain
+// of some 150 float64 instructions, three rows on a warp three times that on
+// one float64 pipe), and a cell's fields split over up to four threads, since a
+// cell holds fineness^2 particles one after the other. Up to 400 fine
+// particles a side, where this shape and 12 rows meet (us per deposition with
+// its finalize, this shape / 12 rows, plasma displaced by several cells:
+// fineness 1: 161^2 11.4 / 18.6, 441^2 28.2 / 28.4; fineness 3: 121^2 9.9 /
+// 11.6, 161^2 14.7 / 13.7; fineness 4: 81^2 9.2 / 13.7, 161^2 21.3 / 22.7). The
+// threads of the 12-row tiles are fitted to fineness 2, and there the line is
+// 240: 41^2 6.5 / 8.4, 81^2 8.0 / 10.8, 121^2 8.6 / 11.5; 161^2 is still ahead
+// alone, 10.2 / 11.6, but in a batch, where other simulations fill the chip,
+// its larger work shows: 8 simulations of 161^2 to 641^2 1292 us a step
+// against 1266.
+constexpr int DEP_SMALL_ROWS = 4;
+// Threads per cell of that shape (1, 2 or 4), 0 where it does not apply. More
+// threads cost more rounds of the window steps (us with 1 / 2 / 4: fineness 1,
+// 161^2 11.4 / 11.7 / 13.7; fineness 2, 121^2 9.2 / 8.6 / 9.9; fineness 4,
+// 81^2 10.7 / 10.0 / 9.2).
+__host__ __device__ inline int dep_small(const DepositArgs& a) {
+    return a.Nf > (a.fineness == 2 ? 240 : 400) ? 0 : a.fineness <= 1 ? 1 : a.fineness <= 3 ? 2 : 4;
+}
 
 // Staged particle of column `col` of a row: even columns, then odd ones, at a
 // pitch of 36. Lanes of neighbouring cells read every other column, lanes of a
@@ -493,9 +517,10 @@ __device__ __forceinline__ double2 coarse_pair(const DepositArgs& a, int k, int 
     }
 }
 
-template <int TI>
+// TI fine rows, RPW of them per warp, FS threads per cell.
+template <int TI, int RPW = 3, int FS = 1>
 __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, int tile_y) {
-    constexpr int T = dep_threads(TI), P = TI * DEP_ROW;
+    constexpr int T = dep_threads(TI, RPW), P = TI * DEP_ROW;
     static_assert(TI <= 32, "masks of 32 bits");
     extern __shared__ __align__(16) double smem_f64[];
     double2* s_pos = reinterpret_cast<double2*>(smem_f64);               // [P] cell offsets
@@ -506,7 +531,7 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
     unsigned* s_mask = reinterpret_cast<unsigned*>(s_R + dep_table_words<TI>());   // [TI][DEP_CELLS]
     unsigned* s_rows = s_mask + TI * DEP_CELLS;                          // [DEP_CELLS]
     __shared__ int s_bb[4];                                              // imin imax jmin jmax
-    const int t = threadIdx.x, lane = t & 31, row0 = (t >> 5) * DEP_RPW;
+    const int t = threadIdx.x, lane = t & 31, row0 = (t >> 5) * RPW;
     if (t == 0) {
         s_bb[0] = s_bb[2] = 1 << 30;
         s_bb[1] = s_bb[3] = -(1 << 30);
@@ -522,11 +547,11 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
     // ---- phase 1 ----
     const int fi0 = tile_y * TI - a.fine_off + row0, fj = tile_x * DEP_TW - a.fine_off + lane;
     const bool col_ok = fj >= 0 && fj < a.Nf;
-    int pi[DEP_RPW], ni[DEP_RPW], pj = 0, nj = 0;
-    double ipi[DEP_RPW], ini[DEP_RPW], fgi[DEP_RPW], ipj = 0, inj = 0, fgj = 0;
-    bool row_ok[DEP_RPW];
+    int pi[RPW], ni[RPW], pj = 0, nj = 0;
+    double ipi[RPW], ini[RPW], fgi[RPW], ipj = 0, inj = 0, fgj = 0;
+    bool row_ok[RPW];
 #pragma unroll
-    for (int u = 0; u < DEP_RPW; ++u) {
+    for (int u = 0; u < RPW; ++u) {
         const int fi = fi0 + u;
         row_ok[u] = row0 + u < TI && fi >= 0 && fi < a.Nf;
         pi[u] = ni[u] = 0;
@@ -552,9 +577,9 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
     const int c1 = __reduce_max_sync(0xffffffffu, col_ok ? (col_idx ? max(pj, nj) : 1 << 30) : -(1 << 30));
     const int nc = c1 - c0 + 1;
     const bool staged = c0 >= 0 && nc >= 1 && nc <= DEP_CMAX;
-    bool ok[DEP_RPW];
+    bool ok[RPW];
 #pragma unroll
-    for (int u = 0; u < DEP_RPW; ++u) {
+    for (int u = 0; u < RPW; ++u) {
         const bool idx = pi[u] >= 0 && pi[u] < a.Nc && ni[u] >= 0 && ni[u] < a.Nc;
         if (row_ok[u] && col_ok && !(idx && col_idx)) raise_flag(a.err, LC3D_FLAG_WINDOW);
         if (!idx) pi[u] = ni[u] = 0;   // nobody uses that row of the table
@@ -564,15 +589,15 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
     if (staged) {
         for (int it = lane; it < nc * 4; it += 32) {
             const int jc = it >> 2, h = it & 3;
-            double2 qp[DEP_RPW], qn[DEP_RPW];
+            double2 qp[RPW], qn[RPW];
 #pragma unroll
-            for (int u = 0; u < DEP_RPW; ++u) {
+            for (int u = 0; u < RPW; ++u) {
                 if (row0 + u >= TI) continue;
                 qp[u] = coarse_pair(a, pi[u] * a.Nc + c0 + jc, h);
                 qn[u] = coarse_pair(a, ni[u] * a.Nc + c0 + jc, h);
             }
 #pragma unroll
-            for (int u = 0; u < DEP_RPW; ++u) {
+            for (int u = 0; u < RPW; ++u) {
                 if (row0 + u >= TI) continue;
                 R[u * DEP_CMAX * 4 + it] = make_double2(ipi[u] * qp[u].x + ini[u] * qn[u].x,
                                                         ipi[u] * qp[u].y + ini[u] * qn[u].y);
@@ -580,15 +605,15 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
         }
     }
     __syncwarp();
-    int cell[DEP_RPW];   // i << 16 | j, or -1
+    int cell[RPW];   // i << 16 | j, or -1
     {
         const int op = (staged && col_ok ? pj - c0 : 0) * 4, on = (staged && col_ok ? nj - c0 : 0) * 4;
-        FineParticle f[DEP_RPW];
+        FineParticle f[RPW];
         bool slow = !staged;
-        double q[DEP_RPW][5];
+        double q[RPW][5];
         if (staged) {
 #pragma unroll
-            for (int u = 0; u < DEP_RPW; ++u) {
+            for (int u = 0; u < RPW; ++u) {
                 const double2* Ru = R + (row0 + u < TI ? u : 0) * DEP_CMAX * 4;
                 double2 w[4];
 #pragma unroll
@@ -605,21 +630,21 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
                 q[u][4] = a.sf * w[3].x;
             }
 #pragma unroll
-            for (int u = 0; u < DEP_RPW; ++u)
+            for (int u = 0; u < RPW; ++u)
                 if (!particle_values_fast(f[u], q[u][0], q[u][1], q[u][2], q[u][3], q[u][4]) && ok[u]) slow = true;
         }
         if (slow) {
 #pragma unroll 1
-            for (int u = 0; u < DEP_RPW; ++u)
+            for (int u = 0; u < RPW; ++u)
                 if (u == 0 ? ok[0] : u == 1 ? ok[1] : ok[2]) {
                     const FineParticle g = fine_particle(a, fi0 + u, fj);
 #pragma unroll
-                    for (int k = 0; k < DEP_RPW; ++k)
+                    for (int k = 0; k < RPW; ++k)
                         if (k == u) f[k] = g;
                 }
         }
 #pragma unroll
-        for (int u = 0; u < DEP_RPW; ++u) {
+        for (int u = 0; u < RPW; ++u) {
             double xl, yl;
             const int i = tsc_cell_1(f[u].x, N, a.h, a.inv_h, xl), j = tsc_cell_1(f[u].y, N, a.h, a.inv_h, yl);
             const bool in = i >= 1 && i <= N - 2 && j >= 1 && j <= N - 2;
@@ -639,7 +664,7 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
     }
     int imin = 1 << 30, imax = -(1 << 30), jmin = 1 << 30, jmax = -(1 << 30);
 #pragma unroll
-    for (int u = 0; u < DEP_RPW; ++u) {
+    for (int u = 0; u < RPW; ++u) {
         if (cell[u] < 0) continue;
         const int i = cell[u] >> 16, j = cell[u] & 0xffff;
         imin = min(imin, i);
@@ -682,7 +707,7 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
             __syncthreads();
         }
 #pragma unroll
-        for (int u = 0; u < DEP_RPW; ++u) {
+        for (int u = 0; u < RPW; ++u) {
             if (cell[u] < 0) continue;
             const int row = row0 + u, i = (cell[u] >> 16) - oi, j = (cell[u] & 0xffff) - oj;
             if (i >= 0 && i < mi && j < mj) {
@@ -706,52 +731,123 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
         }
         __syncthreads();   // masks complete, window cleared
 
-        // ---- phase 2: one cell per thread ----
-        for (int r0 = 0; r0 < ncell; r0 += T) {
-            const int c = r0 + t;
-            unsigned rows = c < ncell ? s_rows[c] : 0u, m = 0;
-            const bool any = rows != 0;
-            const unsigned* mk = s_mask + c;
-            int base = 0;
-            double acc[4][9];
-#pragma unroll
-            for (int f = 0; f < 4; ++f)
-#pragma unroll
-                for (int e = 0; e < 9; ++e) acc[f][e] = 0.0;
-            while (rows | m) {
-                if (!m) {
-                    const int r = __ffs(rows) - 1;
-                    rows &= rows - 1;
-                    m = mk[r * DEP_CELLS];
-                    base = r * DEP_ROW;
-                }
-                const int k = base + dep_slot(__ffs(m) - 1);
-                m &= m - 1;
-                const double2 pos = s_pos[k], v01 = s_v01[k], v23 = s_v23[k];
-                double wx[3], wy[3];
-                tsc_axis(pos.x, wx[0], wx[1], wx[2]);
-                tsc_axis(pos.y, wy[0], wy[1], wy[2]);
-                const double v[4] = {v01.x, v01.y, v23.x, v23.y};
+        // ---- phase 2 ----
+        // One cell per thread written out (as the general form's FS = 1 it
+        // measured 1 to 2 % slower: a run step at 161^2 77.6 us against 76.2).
+        if constexpr (FS == 1) {
+            for (int r0 = 0; r0 < ncell; r0 += T) {
+                const int c = r0 + t;
+                unsigned rows = c < ncell ? s_rows[c] : 0u, m = 0;
+                const bool any = rows != 0;
+                const unsigned* mk = s_mask + c;
+                int base = 0;
+                double acc[4][9];
 #pragma unroll
                 for (int f = 0; f < 4; ++f)
 #pragma unroll
-                    for (int di = 0; di < 3; ++di) {
-                        const double vx = v[f] * wx[di];
-#pragma unroll
-                        for (int dj = 0; dj < 3; ++dj) acc[f][di * 3 + dj] = fma(vx, wy[dj], acc[f][di * 3 + dj]);
+                    for (int e = 0; e < 9; ++e) acc[f][e] = 0.0;
+                while (rows | m) {
+                    if (!m) {
+                        const int r = __ffs(rows) - 1;
+                        rows &= rows - 1;
+                        m = mk[r * DEP_CELLS];
+                        base = r * DEP_ROW;
                     }
-            }
-            const int ci = __float2int_rz(((float)c + 0.5f) * inv_mj), cj = c - ci * mj;
-            double2* w = s_win + ci * wj + cj;
+                    const int k = base + dep_slot(__ffs(m) - 1);
+                    m &= m - 1;
+                    const double2 pos = s_pos[k], v01 = s_v01[k], v23 = s_v23[k];
+                    double wx[3], wy[3];
+                    tsc_axis(pos.x, wx[0], wx[1], wx[2]);
+                    tsc_axis(pos.y, wy[0], wy[1], wy[2]);
+                    const double v[4] = {v01.x, v01.y, v23.x, v23.y};
 #pragma unroll
-            for (int e = 0; e < 9; ++e) {
-                if (any) {
-                    double2* we = w + (e / 3) * wj + e % 3;
-                    const double2 x = we[0], y = we[DEP_WIN];
-                    we[0] = make_double2(x.x + acc[0][e], x.y + acc[1][e]);
-                    we[DEP_WIN] = make_double2(y.x + acc[2][e], y.y + acc[3][e]);
+                    for (int f = 0; f < 4; ++f)
+#pragma unroll
+                        for (int di = 0; di < 3; ++di) {
+                            const double vx = v[f] * wx[di];
+#pragma unroll
+                            for (int dj = 0; dj < 3; ++dj) acc[f][di * 3 + dj] = fma(vx, wy[dj], acc[f][di * 3 + dj]);
+                        }
                 }
-                __syncthreads();
+                const int ci = __float2int_rz(((float)c + 0.5f) * inv_mj), cj = c - ci * mj;
+                double2* w = s_win + ci * wj + cj;
+#pragma unroll
+                for (int e = 0; e < 9; ++e) {
+                    if (any) {
+                        double2* we = w + (e / 3) * wj + e % 3;
+                        const double2 x = we[0], y = we[DEP_WIN];
+                        we[0] = make_double2(x.x + acc[0][e], x.y + acc[1][e]);
+                        we[DEP_WIN] = make_double2(y.x + acc[2][e], y.y + acc[3][e]);
+                    }
+                    __syncthreads();
+                }
+            }
+        } else {   // FS threads per cell, 4 / FS fields each
+            constexpr int NF = 4 / FS;
+            for (int r0 = 0; r0 < ncell * FS; r0 += T) {
+                const int c = (r0 + t) / FS, f0 = (r0 + t) % FS * NF;   // cell, first field
+                unsigned rows = c < ncell ? s_rows[c] : 0u, m = 0;
+                const bool any = rows != 0;
+                const unsigned* mk = s_mask + c;
+                const double2* sv = s_v01 + (f0 >> 1) * P;
+                int base = 0;
+                double acc[NF][9];
+#pragma unroll
+                for (int f = 0; f < NF; ++f)
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) acc[f][e] = 0.0;
+                while (rows | m) {
+                    if (!m) {
+                        const int r = __ffs(rows) - 1;
+                        rows &= rows - 1;
+                        m = mk[r * DEP_CELLS];
+                        base = r * DEP_ROW;
+                    }
+                    const int k = base + dep_slot(__ffs(m) - 1);
+                    m &= m - 1;
+                    const double2 pos = s_pos[k];
+                    double v[NF];
+                    if constexpr (NF == 1) {
+                        v[0] = f0 & 1 ? sv[k].y : sv[k].x;
+                    } else {
+                        double2 x[NF / 2];
+#pragma unroll
+                        for (int h = 0; h < NF / 2; ++h) x[h] = sv[h * P + k];
+#pragma unroll
+                        for (int f = 0; f < NF; ++f) v[f] = f & 1 ? x[f / 2].y : x[f / 2].x;
+                    }
+                    double wx[3], wy[3];
+                    tsc_axis(pos.x, wx[0], wx[1], wx[2]);
+                    tsc_axis(pos.y, wy[0], wy[1], wy[2]);
+#pragma unroll
+                    for (int f = 0; f < NF; ++f)
+#pragma unroll
+                        for (int di = 0; di < 3; ++di) {
+                            const double vx = v[f] * wx[di];
+#pragma unroll
+                            for (int dj = 0; dj < 3; ++dj) acc[f][di * 3 + dj] = fma(vx, wy[dj], acc[f][di * 3 + dj]);
+                        }
+                }
+                const int ci = __float2int_rz(((float)c + 0.5f) * inv_mj), cj = c - ci * mj;
+                double2* w = s_win + (f0 >> 1) * DEP_WIN + ci * wj + cj;
+#pragma unroll
+                for (int e = 0; e < 9; ++e) {
+                    if (any) {
+                        double2* we = w + (e / 3) * wj + e % 3;
+                        if constexpr (NF == 1) {
+                            double& x = f0 & 1 ? we->y : we->x;
+                            x += acc[0][e];
+                        } else {
+                            double2 x[NF / 2];
+#pragma unroll
+                            for (int h = 0; h < NF / 2; ++h) x[h] = we[h * DEP_WIN];
+#pragma unroll
+                            for (int h = 0; h < NF / 2; ++h)
+                                we[h * DEP_WIN] = make_double2(x[h].x + acc[2 * h][e], x[h].y + acc[2 * h + 1][e]);
+                        }
+                    }
+                    __syncthreads();
+                }
             }
         }
 
@@ -770,17 +866,20 @@ __device__ __forceinline__ void deposit_tile(const DepositArgs& a, int tile_x, i
     }
 }
 
-// One tile per CTA: blockIdx.x / .y = tile column / row.
-template <int TI>
-__global__ void __launch_bounds__(dep_threads(TI), 512 / dep_threads(TI)) deposit_kernel(DepositArgs a) {
-    deposit_tile<TI>(a, blockIdx.x, blockIdx.y);
+// One tile per CTA: blockIdx.x / .y = tile column / row. 16 warps per SM, the
+// split cells' smaller patches 24.
+template <int TI, int RPW = 3, int FS = 1>
+__global__ void __launch_bounds__(dep_threads(TI, RPW), (FS > 1 ? 768 : 512) / dep_threads(TI, RPW))
+    deposit_kernel(DepositArgs a) {
+    deposit_tile<TI, RPW, FS>(a, blockIdx.x, blockIdx.y);
 }
 
 // Depositions of several simulations in one launch: CTA b takes the tile
 // b - cta_start[s] of simulation s (cta_start: prefix sums of the tile
-// counts, n + 1 entries), whose arguments are args[s].
-template <int TI>
-__global__ void __launch_bounds__(dep_threads(TI), 512 / dep_threads(TI))
+// counts, n + 1 entries), whose arguments are args[s]. Each simulation's tiles
+// have the shape a launch of its own would give them.
+static_assert(dep_threads(LC3D_DEP_ROWS) == dep_threads(DEP_SMALL_ROWS, 1), "one CTA size for all simulations");
+__global__ void __launch_bounds__(dep_threads(LC3D_DEP_ROWS), 512 / dep_threads(LC3D_DEP_ROWS))
     deposit_multi_kernel(const DepositArgs* __restrict__ args, const int* __restrict__ cta_start, int n) {
     __shared__ DepositArgs sa;
     __shared__ int s_sim;
@@ -802,7 +901,12 @@ __global__ void __launch_bounds__(dep_threads(TI), 512 / dep_threads(TI))
     __syncthreads();
     const int t = (int)blockIdx.x - cta_start[s_sim];
     const int ntx = (sa.Nf + sa.fine_off + DEP_TW - 1) / DEP_TW;
-    deposit_tile<TI>(sa, t % ntx, t / ntx);
+    switch (dep_small(sa)) {
+        case 0: deposit_tile<LC3D_DEP_ROWS>(sa, t % ntx, t / ntx); break;
+        case 1: deposit_tile<DEP_SMALL_ROWS, 1, 1>(sa, t % ntx, t / ntx); break;
+        case 2: deposit_tile<DEP_SMALL_ROWS, 1, 2>(sa, t % ntx, t / ntx); break;
+        default: deposit_tile<DEP_SMALL_ROWS, 1, 4>(sa, t % ntx, t / ntx); break;
+    }
 }
 
 // Accumulators -> float64 (+ ion background), two cells per thread; the
@@ -886,13 +990,38 @@ int launch_move_smart(const MoveArgs& a, cudaStream_t s) {
     return LC3D_OK;
 }
 
+namespace {
+
+// Rows of a tile at its default shape.
+int dep_default_rows(const DepositArgs& a) { return dep_small(a) ? DEP_SMALL_ROWS : LC3D_DEP_ROWS; }
+
+template <int TI, int RPW = 3, int FS = 1>
+int prepare_deposit() {
+    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<TI, RPW, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)dep_smem<TI>()));
+    return LC3D_OK;
+}
+
+template <int TI, int RPW = 3, int FS = 1>
+int launch_deposit(const DepositArgs& a, cudaStream_t s) {
+    const dim3 grid((a.Nf + a.fine_off + DEP_TW - 1) / DEP_TW, (a.Nf + a.fine_off + TI - 1) / TI);
+    LC3D_CUDA_TRY(launch_pdl(deposit_kernel<TI, RPW, FS>, grid, dim3(dep_threads(TI, RPW)), dep_smem<TI>(), s, a));
+    LC3D_CUDA_TRY(cudaGetLastError());
+    return LC3D_OK;
+}
+
+}  // namespace
+
 int particles_prepare() {
-    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep_smem<4>()));
-    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep_smem<8>()));
-    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep_smem<12>()));
-    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dep_smem<16>()));
-    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_multi_kernel<DEP_MULTI_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)dep_smem<DEP_MULTI_ROWS>()));
+    LC3D_TRY(prepare_deposit<4>());
+    LC3D_TRY(prepare_deposit<8>());
+    LC3D_TRY(prepare_deposit<LC3D_DEP_ROWS>());
+    LC3D_TRY(prepare_deposit<16>());
+    LC3D_TRY((prepare_deposit<DEP_SMALL_ROWS, 1, 1>()));
+    LC3D_TRY((prepare_deposit<DEP_SMALL_ROWS, 1, 2>()));
+    LC3D_TRY((prepare_deposit<DEP_SMALL_ROWS, 1, 4>()));
+    LC3D_CUDA_TRY(cudaFuncSetAttribute(deposit_multi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)dep_smem<LC3D_DEP_ROWS>()));
     return LC3D_OK;
 }
 
@@ -910,28 +1039,31 @@ int deposit_fine_offset(int fineness) {
 
 int launch_deposit_main(const DepositArgs& a, cudaStream_t s) {
     if (a.Nf <= 0) return LC3D_OK;
-    const int ti = a.tile_rows ? a.tile_rows : LC3D_DEP_ROWS;
-    const dim3 grid2((a.Nf + a.fine_off + DEP_TW - 1) / DEP_TW, (a.Nf + a.fine_off + ti - 1) / ti);
-    switch (ti) {
-        case 4: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<4>, grid2, dim3(dep_threads(4)), dep_smem<4>(), s, a)); break;
-        case 8: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<8>, grid2, dim3(dep_threads(8)), dep_smem<8>(), s, a)); break;
-        case 12: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<12>, grid2, dim3(dep_threads(12)), dep_smem<12>(), s, a)); break;
-        case 16: LC3D_CUDA_TRY(launch_pdl(deposit_kernel<16>, grid2, dim3(dep_threads(16)), dep_smem<16>(), s, a)); break;
+    switch (a.tile_rows) {
+        case 0: break;
+        case 4: return launch_deposit<4>(a, s);
+        case 8: return launch_deposit<8>(a, s);
+        case 16: return launch_deposit<16>(a, s);
         default: return LC3D_ERR_PARAM;
     }
-    LC3D_CUDA_TRY(cudaGetLastError());
-    return LC3D_OK;
+    switch (dep_small(a)) {
+        case 0: return launch_deposit<LC3D_DEP_ROWS>(a, s);
+        case 1: return launch_deposit<DEP_SMALL_ROWS, 1, 1>(a, s);
+        case 2: return launch_deposit<DEP_SMALL_ROWS, 1, 2>(a, s);
+        default: return launch_deposit<DEP_SMALL_ROWS, 1, 4>(a, s);
+    }
 }
 
-// Tiles of one simulation's deposition at the multi-simulation tile height.
+// Tiles of one simulation's deposition at its default shape.
 int deposit_multi_tiles(const DepositArgs& a) {
-    return ((a.Nf + a.fine_off + DEP_TW - 1) / DEP_TW) * ((a.Nf + a.fine_off + DEP_MULTI_ROWS - 1) / DEP_MULTI_ROWS);
+    const int rows = dep_default_rows(a);
+    return ((a.Nf + a.fine_off + DEP_TW - 1) / DEP_TW) * ((a.Nf + a.fine_off + rows - 1) / rows);
 }
 
 int launch_deposit_multi(const DepositArgs* args_dev, const int* cta_start_dev, int n, int ctas, cudaStream_t s) {
     if (n <= 0 || ctas <= 0) return LC3D_OK;
-    deposit_multi_kernel<DEP_MULTI_ROWS><<<ctas, dep_threads(DEP_MULTI_ROWS), dep_smem<DEP_MULTI_ROWS>(), s>>>(
-        args_dev, cta_start_dev, n);
+    static_assert(dep_smem<LC3D_DEP_ROWS>() >= dep_smem<DEP_SMALL_ROWS>(), "room for either shape");
+    deposit_multi_kernel<<<ctas, dep_threads(LC3D_DEP_ROWS), dep_smem<LC3D_DEP_ROWS>(), s>>>(args_dev, cta_start_dev, n);
     LC3D_CUDA_TRY(cudaGetLastError());
     return LC3D_OK;
 }
@@ -1035,6 +1167,7 @@ extern "C" int lc3d_deposit_noalloc(const lc3d_params* p, const double* ro_initi
     a.acc = scratch;
     a.plane = plane;
     a.Nc = Nc; a.Nf = Nf; a.N = N;
+    a.fineness = p->plasma_fineness;
     a.fine_off = deposit_fine_offset(p->plasma_fineness);
     a.h = p->grid_step_size;
     a.inv_h = 1.0 / p->grid_step_size;

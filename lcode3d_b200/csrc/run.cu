@@ -339,6 +339,7 @@ int batch_capture_multi(lc3d_batch* b, int ph) {
         lc3d_ctx* c = b->c[i];
         DepositArgs t{};
         t.Nf = c->Nf;
+        t.fineness = c->p.plasma_fineness;
         t.fine_off = deposit_fine_offset(c->p.plasma_fineness);
         start[i + 1] = start[i] + deposit_multi_tiles(t);
         memset(c->graph_launches[b->par0[i] ^ ph], 0, sizeof(c->graph_launches[0]));   // gathered over segments

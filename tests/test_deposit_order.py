@@ -72,7 +72,7 @@ MAIN = r'''
 static DepositArgs g_args;
 static int g_tx, g_ty;
 static void body() {
-    deposit_tile<TI>(g_args, g_tx, g_ty);
+    deposit_tile<TI, RPW, FS>(g_args, g_tx, g_ty);
     g_state[g_now] = 3;
     swapcontext(&g_ctx[g_now], &g_main);
 }
@@ -125,7 +125,7 @@ int main(int argc, char** argv) {
     std::vector<int32_t> ip(Nf), in(Nf);
     if (fread(ip.data(), 4, Nf, f) != (size_t)Nf || fread(in.data(), 4, Nf, f) != (size_t)Nf) return 1;
     fclose(f);
-    g_threads = dep_threads(TI);
+    g_threads = dep_threads(TI, RPW);
     std::vector<std::vector<char>> stacks(g_threads, std::vector<char>(65536));
     FILE* o = fopen(argv[2], "wb");
     for (int order = 0; order < 2; ++order) {
@@ -157,7 +157,7 @@ int main(int argc, char** argv) {
 '''
 
 
-def program(tmp_path, rows):
+def program(tmp_path, rows, per_warp, split):
     src = open(f'{ROOT}/lcode3d_b200/csrc/particles.cu').read()
     args = re.search(r'struct DepositArgs \{.*?\n\};\n', open(f'{ROOT}/lcode3d_b200/csrc/lc3d_internal.cuh').read(), re.S).group(0)
     body = src[src.index('struct Tsc {'):src.index('// Field-free estimate')]
@@ -167,14 +167,14 @@ def program(tmp_path, rows):
     body = re.sub(r'asm\("rcp\.approx.*', 'r = 1 / d;', body)
     body = re.sub(r'extern __shared__ .*\n', '', body)
     cpp = tmp_path / 'deposit.cpp'
-    cpp.write_text(SHIM + 'alignas(16) static double smem_f64[29056];\n' + args + body + f'#define TI {rows}\n' + MAIN)
+    cpp.write_text(SHIM + 'alignas(16) static double smem_f64[29056];\n' + args + body + f'#define TI {rows}\n#define RPW {per_warp}\n#define FS {split}\n' + MAIN)
     exe = tmp_path / 'deposit'
     subprocess.run(['g++', '-O1', '-std=c++17', '-w', '-o', str(exe), str(cpp)], check=True)
     return exe
 
 
-@pytest.mark.parametrize('rows', [12, 4])
-def test_deposit_does_not_depend_on_the_order_of_warps(tmp_path, rows):
+@pytest.mark.parametrize('rows, per_warp, split', [(12, 3, 1), (4, 3, 1), (4, 1, 1), (4, 1, 2), (4, 1, 4)])
+def test_deposit_does_not_depend_on_the_order_of_warps(tmp_path, rows, per_warp, split):
     N, coarse, fine = 41, 3, 2
     cfg = make_config(N, 0.1, 0.05, 10, amplitude=0.3)
     x0, y0, *_, m, q, virt = O.make_plasma(N - 2 * cfg.plasma_padding_steps, 0.1, coarse, fine)
@@ -192,7 +192,7 @@ def test_deposit_does_not_depend_on_the_order_of_warps(tmp_path, rows):
         for a in (virt.indices_prev, virt.indices_next):
             np.ascontiguousarray(a, dtype=np.int32).tofile(f)
     out = tmp_path / 'out'
-    subprocess.run([str(program(tmp_path, rows)), str(data), str(out)], check=True, timeout=300)
+    subprocess.run([str(program(tmp_path, rows, per_warp, split)), str(data), str(out)], check=True, timeout=300)
     raw = out.read_bytes()
     size = 4 * N * N * 8 + 12
     orders = [np.frombuffer(raw[k * size:k * size + size - 12]).reshape(4, N, N) for k in range(2)]

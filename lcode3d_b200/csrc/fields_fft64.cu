@@ -65,7 +65,7 @@ struct F64Field {
     double* partial;        // B, Bz: this field's sums per CTA; D: the same, to be read
     int npartial;
     const int* tab;         // A: row p of out at [q NB + b], or -1; D: column p of in, top bit: negated
-    int border;             // D: the first and last grid rows are zero
+    int border;             // axis 0 antisymmetric; A: the first grid row is not read; D: the first and last are zero
     int zero;               // D: a column of zeros in `in`
     const double* prev;     // D: step finalize
     double* avg;
@@ -460,13 +460,15 @@ __device__ __forceinline__ const F64Field& field_of(const F64Batch& b, int cta) 
 
 // First pass of A and B: pairs of rows of `in`, column c the transform's
 // element c (0 .. L). Rows past the end repeat the last one (what comes of
-// them goes to columns nobody reads). ROTATE (A, which is not transformed
+// them goes to columns nobody reads). The first grid row of an antisymmetric
+// axis 0 is not read either, the second stands in for it: its values are no part
+// of the field, and as one of a pair they would reach the other row. ROTATE (A, which is not transformed
 // back): an antisymmetric pair is read as i z, so that its transform is
 // (X_a, X_b) as it stands; B leaves the factors of i and -1 to Lambda.
 template <int R1, bool ROTATE, int LF>
 __device__ __forceinline__ void load_rows(const Shared<LF>& S, const F64Plan& p, const double2* tw, const F64Field& F, int row0) {
     first_pass<R1>(S, p, tw, F.type, [&](int f, int j, double2 (&v)[R1]) {
-        const int ra = min(row0 + 2 * f, F.rows - 1), rb = min(row0 + 2 * f + 1, F.rows - 1);
+        const int ra = max(min(row0 + 2 * f, F.rows - 1), F.border), rb = min(row0 + 2 * f + 1, F.rows - 1);
         const bool rot = ROTATE && F.type;
         const double* x = F.in + (ptrdiff_t)(rot ? rb : ra) * F.ld_in;
         const double* y = F.in + (ptrdiff_t)(rot ? ra : rb) * F.ld_in;
@@ -960,10 +962,11 @@ int fft64_solve(lc3d_ctx* c, const Fft64Desc* desc, int count, cudaStream_t s) {
             f.cta_start = ctas;
             f.ld_out = st->pitch;
             int rows = N;
-            if (pass == 0) {        // all grid rows: a border row of an antisymmetric axis 0 is read by nobody
+            if (pass == 0) {        // all grid rows: what comes of an antisymmetric axis 0's border rows is read by nobody
                 f.in = d.rhs; f.ld_in = N; f.rows = N; f.type = d.type1;
                 f.out = d.t1;
                 f.tab = tab_a(st, d.type1);
+                f.border = d.type0;
             } else if (pass == 1) {
                 f.in = d.t1; f.ld_in = st->pitch; f.rows = rows = n1; f.type = d.type0;
                 f.out = d.t2;

@@ -64,7 +64,8 @@ __device__ __forceinline__ void sqrt_fast(double S, double& g, double& inv) {
 }
 __device__ __forceinline__ bool in_fast_range(double S) { return S > 0x1p-900 && S < 0x1p900; }
 
-// 1 / d by Newton's iteration, for a quotient x / d = div_h(x, d, recip_fast(d)).
+// 1 / d by Newton's iteration, for a quotient x / d = div_h(x, d, recip_fast(d));
+// d not 0.
 __device__ __forceinline__ double recip_fast(double d) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
@@ -133,11 +134,12 @@ __device__ __forceinline__ void estimate_one(double m, double xi0, double yi0, d
                                              double& ex, double& ey) {
     double x = xi0 + xo, y = yi0 + yo;
     const double S = m * m + pz * pz + px * px + py * py;
+    double gamma_f, inv;
+    sqrt_fast(S, gamma_f, inv);
+    const double d = gamma_f - pz;
     double vx, vy;
-    if (in_fast_range(S)) {
-        double gamma_m, inv;
-        sqrt_fast(S, gamma_m, inv);
-        const double d = gamma_m - pz, r = recip_fast(d);
+    if (in_fast_range(S) && d != 0) {   // 0: pz swamps the rest
+        const double r = recip_fast(d);
         vx = div_h(px, d, r);
         vy = div_h(py, d, r);
     } else {
@@ -182,7 +184,8 @@ __device__ __forceinline__ void store_packed(double* p, double x, double y, doub
 // its time in this chain: 80.1 -> 79.0 us per xi step without the branches, 81^2
 // 74 -> 69, 641^2 363 -> 361): two passes from the old momenta in the
 // gathered fields, then the velocity of the half-way momenta. FAST: without
-// branches (sqrt_fast); returns false if a square root left its range.
+// branches (sqrt_fast); returns false if a square root left its range or the
+// last quotients' denominator is 0 (1 - vz = 0 makes the next square root NaN).
 struct Push {
     double px, py, pz, dpx, dpy, dpz, vx, vy;   // half-way momenta, changes, dx / dxi, dy / dxi
 };
@@ -205,6 +208,7 @@ __device__ __forceinline__ bool push(double m, double q, double dxi, double opx,
         if (it == 2) {
             const double d = gamma_m - pz;
             if (FAST) {
+                ok = ok && d != 0;   // 0: pz swamps the rest
                 const double r = recip_fast(d);
                 o.vx = div_h(px, d, r);
                 o.vy = div_h(py, d, r);

@@ -2,6 +2,8 @@
 // per-stage entry points. Reference: lcode.py:828-931 (step), 936-975
 // (init), and the stage functions cited in include/lc3d.h.
 
+#include <cudaTypedefs.h>
+
 #include <cstdlib>
 #include <cstring>
 #include <new>
@@ -121,16 +123,42 @@ __global__ void __launch_bounds__(256) copy_state_kernel(const __grid_constant__
     }
 }
 
-// Whether a kernel on `device` may access p: its own memory or managed
-// memory. The runtime copies from and to other memory (a peer's), or refuses
-// the pointer, which a kernel cannot.
-bool on_device(const void* p, int device) {
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+// Whether copy_state_kernel may stand for the 15 copies from or to a caller's
+// arrays: whole, aligned elements, each array inside one allocation of this
+// device (or managed), no two that overlap if they are written. The runtime's copies take any
+// alignment, keep their order where arrays overlap, reach host and peer memory,
+// and refuse what is no memory, all of which a kernel cannot.
+bool kernel_may_copy(const double* const* p, size_t np, size_t ng, int device, bool written) {
+    static const PFN_cuMemGetAddressRange_v3020 range_of = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool ok = cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) == cudaSuccess &&
+                        q == cudaDriverEntryPointSuccess;
+        return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(ok ? f : nullptr);
+    }();
+    if (!range_of) return false;
+    CUdeviceptr base = 0;   // the allocation of the array before: often all are views of one
+    size_t size = 0;
+    for (int k = 0; k < 15; ++k) {
+        const uintptr_t at = reinterpret_cast<uintptr_t>(p[k]);
+        const size_t bytes = (k < 5 ? np : ng) * sizeof(double);
+        if (at % sizeof(double)) return false;
+        if (!(at >= base && at - base < size)) {
+            cudaPointerAttributes a{};
+            if (cudaPointerGetAttributes(&a, p[k]) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            if (!((a.type == cudaMemoryTypeDevice && a.device == device) || a.type == cudaMemoryTypeManaged)) return false;
+            if (range_of(&base, &size, (CUdeviceptr)at) != CUDA_SUCCESS) return false;
+        }
+        if (at < base || bytes > size || at - base > size - bytes) return false;
+        for (int j = 0; written && j < k; ++j) {
+            const uintptr_t other = reinterpret_cast<uintptr_t>(p[j]);
+            if (at < other + (j < 5 ? np : ng) * sizeof(double) && other < at + bytes) return false;
+        }
     }
-    return (at.type == cudaMemoryTypeDevice && at.device == device) || at.type == cudaMemoryTypeManaged;
+    return true;
 }
 
 int copy_state(const lc3d_state_ptrs& dst, const lc3d_state_ptrs& src, size_t np, size_t ng, const lc3d_ctx* c,
@@ -141,11 +169,10 @@ int copy_state(const lc3d_state_ptrs& dst, const lc3d_state_ptrs& src, size_t np
                          src.Bx, src.By, src.Bz, src.ro, src.jx, src.jy, src.jz}, np, ng};
     for (int k = 0; k < 15; ++k)
         if (!a.dst[k] || !a.src[k]) return LC3D_ERR_PARAM;
-    double* const theirs[] = {caller.x_offt, caller.y_offt, caller.px, caller.py, caller.pz, caller.Ex, caller.Ey, caller.Ez,
-                              caller.Bx, caller.By, caller.Bz, caller.ro, caller.jx, caller.jy, caller.jz};
-    bool own = true;
-    for (double* q : theirs) own = own && on_device(q, c->device);
-    if (!own) {
+    const double* const theirs[] = {caller.x_offt, caller.y_offt, caller.px, caller.py, caller.pz,
+                                    caller.Ex, caller.Ey, caller.Ez, caller.Bx, caller.By, caller.Bz,
+                                    caller.ro, caller.jx, caller.jy, caller.jz};
+    if (!kernel_may_copy(theirs, np, ng, c->device, caller.x_offt == dst.x_offt)) {
         for (int k = 0; k < 15; ++k)
             LC3D_CUDA_TRY(cudaMemcpyAsync(a.dst[k], a.src[k], (k < 5 ? np : ng) * sizeof(double),
                                           cudaMemcpyDeviceToDevice, s));

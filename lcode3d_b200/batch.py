@@ -167,14 +167,16 @@ def _time_sim(spec, precision, form, tiles, steps):
     return e0.elapsed_time(e1) / steps
 
 
-TILE_CHOICES = {'deposit_rows': (4, 8, 16), 'fft_ctas_per_sm': (0, 2)}
+# 0: the default, among them so that a choice is never slower than none
+TILE_CHOICES = {'deposit_rows': (0, 4, 8, 16), 'fft_ctas_per_sm': (0, 2)}
 
 
 def autotune(grids, steps=6, precision='fp64'):
     """Pick, per grid size, the float64 transform form (FFT or dense) and
-    the tile shapes (deposition fine rows per CTA; resident FFT CTAs per SM,
-    0 = as many as fit) by timing a few graph-replayed steps of every
-    combination on this GPU. Returns ({N: {'transform', 'deposit_rows',
+    the tile shapes (deposition fine rows per CTA, 0 = the default; resident
+    CTAs per SM of the float32 FFT passes, 0 = as many as fit) by timing a
+    few graph-replayed steps of every combination on this GPU; one time stands
+    for all FFT settings where the precision has no float32 passes. Returns ({N: {'transform', 'deposit_rows',
     'fft_ctas_per_sm'}}, {N: {label: ms per step}})."""
     choice, timings = {}, {}
     for N in sorted(set(grids)):
@@ -184,8 +186,10 @@ def autotune(grids, steps=6, precision='fp64'):
         best = None
         for form in ('fft', 'dense'):
             for rows in TILE_CHOICES['deposit_rows']:
+                ms = None
                 for per_sm in (TILE_CHOICES['fft_ctas_per_sm'] if form == 'fft' else (0,)):
-                    ms = _time_sim(spec, precision, form, (rows, per_sm), steps)
+                    if ms is None or precision == 'fft32':
+                        ms = _time_sim(spec, precision, form, (rows, per_sm), steps)
                     if ms is None:
                         continue
                     timings[N][f'{form} rows={rows} fft_per_sm={per_sm}'] = ms

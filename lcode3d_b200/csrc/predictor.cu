@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv3x3_tc_kernel(const __gri
     }
     fence_before();
     __syncthreads();
-    if (s_fail && threadIdx.x == 0) atomicOr(a.err, LC3D_FLAG_TIMEOUT);
+    if (s_fail && threadIdx.x == 0) atomicOr(a.err, 1u);
     if (warp == 1) {
         fence_after();
         tmem_dealloc(tmem, tcols);
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_wgrad_tc_kernel(const __
     }
     fence_before();
     __syncthreads();
-    if (s_fail && threadIdx.x == 0) atomicOr(a.err, LC3D_FLAG_TIMEOUT);
+    if (s_fail && threadIdx.x == 0) atomicOr(a.err, 1u);
     if (warp == 1) {
         fence_after();
         tmem_dealloc(tmem, tcols);
@@ -864,7 +864,7 @@ struct lc3d_predictor {
     dim3 wg_grid[NLAYERS];
     cudaStream_t wg_stream = nullptr;              // the weight-gradient passes' stream
     cudaEvent_t ev_grad[NLAYERS] = {}, ev_wg[NLAYERS] = {};   // layer l's g_bf written; read by its weight pass
-    unsigned* err = nullptr;
+    unsigned* err = nullptr;       // device word: a wait ran out (this object's own, not a context's flag words)
     double* scale = nullptr;       // [23] per-sample channel scales (device)
     double* partial = nullptr;     // [STAT_BLOCKS][18]
     double mult[23];               // scale multipliers (host-set)

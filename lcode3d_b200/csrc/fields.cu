@@ -368,11 +368,12 @@ int fields_init(lc3d_ctx* c) {
     for (int i = 0; i < N; ++i)
         for (int j = 0; j < N; ++j)
             ln[(size_t)i * N + j] = (i == 0 && j == 0) ? 0.0 : (1 / (lamk[i] + lamk[j])) * norm;
-    LC3D_TRY(upload(&c->lam_dir, ld));
-    LC3D_TRY(upload(&c->lam_mix, lm));
-    LC3D_TRY(upload(&c->lam_mixT, lmT));
-    LC3D_TRY(upload(&c->lam_neu, ln));
-    if (c->p.precision == LC3D_PREC_FFT32) {
+    if (c->p.precision != LC3D_PREC_FFT32) {
+        LC3D_TRY(upload(&c->lam_dir, ld));
+        LC3D_TRY(upload(&c->lam_mix, lm));
+        LC3D_TRY(upload(&c->lam_mixT, lmT));
+        LC3D_TRY(upload(&c->lam_neu, ln));
+    } else {
         LC3D_TRY(upload32(&c->lam32_dir, ld));
         LC3D_TRY(upload32(&c->lam32_mix, lm));
         LC3D_TRY(upload32(&c->lam32_mixT, lmT));
@@ -384,10 +385,11 @@ int fields_init(lc3d_ctx* c) {
         LC3D_CUDA_TRY(cudaMalloc(&c->rhs[f], plane));
         LC3D_CUDA_TRY(cudaMalloc(&c->t1[f], tplane));
         LC3D_CUDA_TRY(cudaMalloc(&c->t2[f], tplane));
-        LC3D_CUDA_TRY(cudaMalloc(&c->raw[f], plane));
         LC3D_CUDA_TRY(cudaMemset(c->t1[f], 0, tplane));
         LC3D_CUDA_TRY(cudaMemset(c->t2[f], 0, tplane));
         LC3D_CUDA_TRY(cudaMemset(c->rhs[f], 0, plane));
+        if (c->use_fft && c->p.precision == LC3D_PREC_FP64) continue;   // these solves write the fields themselves
+        LC3D_CUDA_TRY(cudaMalloc(&c->raw[f], plane));
         LC3D_CUDA_TRY(cudaMemset(c->raw[f], 0, plane));
     }
     c->red_blocks = 160;
@@ -396,12 +398,18 @@ int fields_init(lc3d_ctx* c) {
     return LC3D_OK;
 }
 
-void fields_free(lc3d_ctx* c) {
-    double** ps[] = {&c->lam_dir, &c->lam_mix, &c->lam_mixT, &c->lam_neu, &c->red};
+void fields_drop_lam(lc3d_ctx* c) {
+    double** ps[] = {&c->lam_dir, &c->lam_mix, &c->lam_mixT, &c->lam_neu};
     for (double** p : ps) {
         if (*p) cudaFree(*p);
         *p = nullptr;
     }
+}
+
+void fields_free(lc3d_ctx* c) {
+    fields_drop_lam(c);
+    if (c->red) cudaFree(c->red);
+    c->red = nullptr;
     float** ps32[] = {&c->lam32_dir, &c->lam32_mix, &c->lam32_mixT, &c->lam32_neu};
     for (float** p : ps32) {
         if (*p) cudaFree(*p);

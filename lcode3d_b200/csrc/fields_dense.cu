@@ -321,21 +321,23 @@ int dense_init(lc3d_ctx* c) {
             };
             const int ld = mat_pitch(n);
             const size_t nn = (size_t)n * ld;
-            std::vector<double> h(4 * nn, 0.0);
+            std::vector<double> h((type ? 2 : 4) * nn, 0.0);   // the DST-I matrix is symmetric: back = forth_t
             for (int k = 0; k < n; ++k)
                 for (int x = 0; x < n; ++x) {
-                    const double f = T(2 * k + q, x), b = T(x, 2 * k + q);
+                    const double f = T(2 * k + q, x);
                     h[(size_t)k * ld + x] = f;
                     h[nn + (size_t)x * ld + k] = f;
+                    if (type) continue;
+                    const double b = T(x, 2 * k + q);
                     h[2 * nn + (size_t)x * ld + k] = b;
                     h[3 * nn + (size_t)k * ld + x] = b;
                 }
             HalfMats& m = d->m[type][q];
-            LC3D_CUDA_TRY(cudaMalloc(&m.forth, 4 * nn * sizeof(double)));
-            LC3D_CUDA_TRY(cudaMemcpy(m.forth, h.data(), 4 * nn * sizeof(double), cudaMemcpyHostToDevice));
+            LC3D_CUDA_TRY(cudaMalloc(&m.forth, h.size() * sizeof(double)));
+            LC3D_CUDA_TRY(cudaMemcpy(m.forth, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
             m.forth_t = m.forth + nn;
-            m.back = m.forth + 2 * nn;
-            m.back_t = m.forth + 3 * nn;
+            m.back = type ? m.forth_t : m.forth + 2 * nn;
+            m.back_t = type ? m.forth : m.forth + 3 * nn;
         }
     const double* src[4] = {c->lam_neu, c->lam_mixT, c->lam_mix, c->lam_dir};
     for (int k = 0; k < 4; ++k) {
@@ -345,6 +347,7 @@ int dense_init(lc3d_ctx* c) {
         lam_parity_kernel<<<dim3((width + 127) / 128, rows), 128>>>(src[k], rows, cols, d->lam[k]);
         LC3D_CUDA_TRY(cudaGetLastError());
     }
+    fields_drop_lam(c);   // this state has its own, sorted by parity
     return LC3D_OK;
 }
 

@@ -926,6 +926,7 @@ int fft64_init(lc3d_ctx* c) {
                                                                     s->lam[k], s->pitch);
         LC3D_CUDA_TRY(cudaGetLastError());
     }
+    fields_drop_lam(c);   // this state has its own, in its order
     for (int pass = 0; pass < 3; ++pass)   // per kernel, not per context: the largest any context may use
         LC3D_CUDA_TRY(cudaFuncSetAttribute(kernel_of(pass, p.lf), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)F64_MAX_SMEM));

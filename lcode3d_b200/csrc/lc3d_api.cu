@@ -706,15 +706,15 @@ int lc3d_create(const lc3d_params* p, int device, lc3d_ctx** out) {
     if (rc == LC3D_OK && cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess) rc = LC3D_ERR_CUDA;
     try {   // tables built in host memory
         LC3D_STEP(particles_prepare());
-        LC3D_STEP(fields_init(c));
         LC3D_STEP(fft_init(c));
-        LC3D_STEP(run_init(c));
-        LC3D_STEP(diag_init(c));
         if (rc == LC3D_OK) {
             if (p->fp64_transform == LC3D_FP64_FFT && !c->fft_ok) rc = LC3D_ERR_PARAM;
             if (p->precision == LC3D_PREC_FFT32 && !c->fft_ok) rc = LC3D_ERR_PARAM;   // no dense float32 form
             c->use_fft = c->fft_ok && p->fp64_transform != LC3D_FP64_DENSE;
         }
+        LC3D_STEP(fields_init(c));
+        LC3D_STEP(run_init(c));
+        LC3D_STEP(diag_init(c));
         if (p->precision == LC3D_PREC_FP64) LC3D_STEP(c->use_fft ? fft64_init(c) : dense_init(c));
         if (p->precision == LC3D_PREC_MIXED) LC3D_STEP(mixed_init(c, p->mixed_slices ? p->mixed_slices : 4, 0));
         if (p->precision == LC3D_PREC_TF32) LC3D_STEP(mixed_init(c, p->mixed_slices ? p->mixed_slices : 3, 1));

@@ -266,7 +266,8 @@ int mixed_stage(lc3d_ctx* ctx, const MixedStageDesc* d, int count, cudaStream_t 
 // one-time per-device kernel attributes (shared-memory opt-ins)
 int particles_prepare();
 int fft_prepare(int P);
-int fields_init(lc3d_ctx* ctx);           // transform matrices, workspaces
+int fields_init(lc3d_ctx* ctx);           // eigenvalue matrices, workspaces (after use_fft is set)
+void fields_drop_lam(lc3d_ctx* ctx);      // the float64 eigenvalue matrices, once a solver has its own
 int diag_init(lc3d_ctx* ctx);             // diagnostics.cu
 void diag_free(lc3d_ctx* ctx);
 void fields_free(lc3d_ctx* ctx);

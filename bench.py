@@ -403,9 +403,9 @@ def run_ours(args, rank, world, dist):
                 'traffic': None,
                 'note': ('the rows stay in L2 (ncu: L2 throughput ~0.14 of peak); while active the pass is '
                          'bound by the L1/shared-memory pipe (~0.72 of peak) and by its barrier-separated radix '
-                         'passes: profiles/fft_rows_kernel_641.md') if f32 else
+                         'passes') if f32 else
                         ('the rows stay in L2 (ncu: L2 throughput ~0.11 of peak); bound by latency: FP64 pipe '
-                         '~0.22, issue ~0.27 of peak at 16 warps per SM: profiles/fft64_kernels_641.md')}
+                         '~0.22, issue ~0.27 of peak at 16 warps per SM')}
     elif dom == 'transform' and stage[dom]['timed']:
         avg_ms = stage[dom]['ms'] / stage[dom]['timed']
         fl = transform_flops_per_launch(N) / 2 * 4 / 6   # half-size matrices; 4 of a solve's 6 launches are GEMMs
@@ -641,7 +641,7 @@ def run_scan(args, rank, world, dist):
         'data': 'synthetic (seeded scan draws, generated plasma and beams)',
         'config': {'workload': f'{len(specs)} independent simulations, grids {counts}, window +-8, dxi 0.01',
                    'seed': args.seed, 'l2': 'no flush (each batch step touches several GB, far more than L2)',
-                   'deposition': ('one launch over all simulations per deposition point (4-row tiles)' if multi
+                   'deposition': ('one launch over all simulations per deposition point (default tiles)' if multi
                                   else 'per simulation, on its graph branch (autotuned tile rows)')},
         'autotune': {'choice': {str(k): v for k, v in choice.items()},
                      'ms_per_step': {str(k): v for k, v in timings.items()}},

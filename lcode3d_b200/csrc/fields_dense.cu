@@ -101,24 +101,15 @@ __global__ void lam_parity_kernel(const double* __restrict__ lam, int rows, int 
 // sums throughout). 64 x 32 tiles per 128-thread CTA, a 32 x 16 tile (2 x 2
 // MMAs per k8 step) per warp; k-steps of 16 staged by 16-byte cp.async into
 // two shared-memory buffers, the next k-step copied while the current one is
-// multiplied. With copies of 8 bytes, twice as many and each with its address
-// arithmetic, the MMA pipe was 53 % busy; with these an xi step in a
-// graph at 255^2 172 -> 157 us, 387^2 316 -> 292, 641^2 970 -> 911 (rows on 16
-// bytes only 162, 301, 920; past L1, as .cg, 163, 394, 910: the CTAs of an SM
-// share their panels there).
+// multiplied. Copies go through L1 (.ca): the CTAs of an SM share their
+// panels there (an xi step in a graph at 387^2 292 us, past L1 394).
 //
 // The tile is small because the problems are: at 387^2 a launch has 12 of
 // about 387 x 194 x 194, and what is lost is rows and columns past the edges
-// and SMs with a tile less than others. 28 us a launch at 387^2 with 8-byte copies
-// and two warps of 32 x 32; 35 with m8n8k4 MMAs and bounds checks on every
-// copy; 78 with matrices of full size in 128 x 64 tiles. Four warps of 32 x 16
-// a CTA hide more of a k-step's latency than two of 32 x 32 (an xi step in a
-// graph at 43^2 91 -> 80 us, 163^2 128 -> 107, 255^2 157 -> 142, 431^2 370 ->
-// 350, 513^2 495 -> 482, 641^2 911 -> 772; 387^2 292 -> 297); five CTAs per SM
-// instead of six 524 at 513^2. Leaving out the MMAs past the edges (a fifth
-// of a launch's at 387^2) was slower, for the branches: 316 -> 340; whole
-// warps left out changed nothing. Tiles of 32 x 64 where they are fewer: 431^2
-// 350 -> 340, but 387^2 297 -> 301.
+// and SMs with a tile less than others (a launch at 387^2 28 us; 78 with
+// matrices of full size in 128 x 64 tiles of m8n8k4 MMAs). Four warps of
+// 32 x 16 a CTA hide more of a k-step's latency than two of 32 x 32: an xi step
+// in a graph at 163^2 107 us against 128, 641^2 772 against 911.
 // ---------------------------------------------------------------------------
 constexpr int MAX_PROBS = 12;
 

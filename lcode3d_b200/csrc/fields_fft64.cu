@@ -848,10 +848,9 @@ int fft64_init(lc3d_ctx* c) {
     // shared memory allows, else 512 threads and one. Eight pairs store whole
     // lines and fill the SMs from about 400 rows on; smaller grids take four,
     // for twice the CTAs, and so do those of 700 to 1100 rows, of which eight
-    // pairs fit an SM once and four twice (us per xi step, F = 8 / F = 4: 161^2
-    // 79.3 / 76.1, 321^2 129.0 / 119.4, 401^2 199 / 222, 641^2 372 / 430; 801^2
-    // 621 / 600, 961^2 800 / 778, 1025^2 927 / 913, 1153^2 1118 / 1156, 1281^2
-    // 1482 / 1549).
+    // pairs fit an SM once and four twice (us per xi step, F = 8 / F = 4, around
+    // the lines: 321^2 129.0 / 119.4, 401^2 199 / 222; 641^2 372 / 430, 801^2
+    // 621 / 600; 1025^2 927 / 913, 1153^2 1118 / 1156).
     auto twice = [&](int lf) {
         p.lf = lf;
         return 2 * (smem_bytes(p) + 2048) <= 228 * 1024;

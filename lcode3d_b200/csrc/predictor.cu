@@ -41,9 +41,10 @@
 // Training: both gradient passes of every convolution on the tensor cores
 // in bf16 -- the data gradient as the forward convolution of the bf16 output
 // gradient with flipped, transposed weights, the weight gradient as an
-// implicit GEMM over pixels with MN-major operands -- and float32 SIMT
-// kernels for the bias gradients, the pooling / upsampling / ReLU adjoints,
-// an MSE loss on the 5 fields and Adam. Weights are kept as float32 master
+// implicit GEMM over pixels with MN-major operands -- and SIMT kernels for an
+// MSE loss on the 5 fields, the pooling / upsampling / ReLU adjoints, which
+// write the output gradients in bf16 and sum the bias gradients on the way,
+// and Adam. Weights are kept as float32 master
 // copies; the bf16 copies the forward pass reads are refreshed after every
 // update.
 
@@ -228,8 +229,8 @@ constexpr size_t conv_smem_bytes(int cout = 128) {
 // group (the next box) LBO = 4 KiB further, 8-pixel row groups SBO = 512 bytes
 // apart. M = 128 output channels, N = Cin.
 // A CTA sums one chunk of pixels for one tap in TMEM (f32) and adds its
-// partial to dW with float32 atomics. The bias gradient stays a plain
-// reduction. Pixels past the level and shifted rows outside it are zero
+// partial to dW with float32 atomics. (The bias gradient comes with g: the
+// gradient kernels below.) Pixels past the level and shifted rows outside it are zero
 // fill; the pad column of g is zero.
 // ---------------------------------------------------------------------------
 constexpr int WG_PIX = 64;                                  // pixels per stage
@@ -609,8 +610,8 @@ __global__ void flip_weights_kernel(const __nv_bfloat16* __restrict__ w, int CG,
 }
 
 // ---------------------------------------------------------------------------
-// Training kernels (float32): bias gradients, pooling / upsampling / ReLU
-// adjoints and Adam
+// Training kernels: loss, pooling / upsampling / ReLU adjoints with the bias
+// gradients, Adam
 // ---------------------------------------------------------------------------
 
 // The kernels that produce a layer's output gradient write it in bf16, the
@@ -853,8 +854,8 @@ struct lc3d_predictor {
     float *y = nullptr, *target = nullptr;
     // gradients (float32 NHWC)
     float *g_d1 = nullptr, *g_d2 = nullptr, *g_e3 = nullptr, *g_p2 = nullptr, *g_p1 = nullptr;
-    // tensor-core backward passes: the bf16 output gradients of two layers, the flipped transposed bf16 weights of every layer, zeros for
-    // the bias, and the convolution arguments of each layer's pass
+    // tensor-core backward passes: the bf16 output gradients of two layers,
+    // the flipped transposed bf16 weights of every layer, zeros for the bias, and the convolution arguments of each layer's pass
     __nv_bfloat16* g_bf[2] = {nullptr, nullptr};   // layer l uses g_bf[l & 1]
     __nv_bfloat16* wt = nullptr;
     long long wt_off[NLAYERS];
